@@ -27,7 +27,8 @@ struct SlabArgs {
   const float2* tw;
   const float* rden;
   int rden_div;
-  float2* cand;  // [item][nb]: (value, bits of index)
+  float2* cand;  // [item][nb]: (value, bits of index); keyed: (~index, ordered value) as one 64-bit key
+  int keyed;
   float* vol;    // volume mode: [item][nb][nc][n]
 };
 
@@ -123,6 +124,7 @@ __global__ void __launch_bounds__(256) k_slab(SlabArgs a) {
 // kept by a strict comparison; lanes then reduce by (value, lowest index).
 template <int N>
 __device__ __forceinline__ float2 tw_of(int t);
+template <> __device__ __forceinline__ float2 tw_of<8>(int t) { return make_float2(kTwRe16[2 * t], kTwIm16[2 * t]); }
 template <> __device__ __forceinline__ float2 tw_of<16>(int t) { return make_float2(kTwRe16[t], kTwIm16[t]); }
 template <> __device__ __forceinline__ float2 tw_of<32>(int t) { return make_float2(kTwRe32[t], kTwIm32[t]); }
 template <> __device__ __forceinline__ float2 tw_of<64>(int t) { return make_float2(kTwRe64[t], kTwIm64[t]); }
@@ -309,6 +311,158 @@ __global__ void __launch_bounds__(WARPS * 32, PER_SM) k_slab_cols(SlabArgs a) {
   }
 }
 
+// ── the slab a block at a time, its transform split over the block's warps ──
+//
+// Where a column's half-length transform (H points) does not fit one lane's registers, or nc columns
+// of rden rows do not fit a warp's share of shared memory, a block of R2/2 warps takes 32 columns of a
+// slab (lane = column) and computes H = R1·R2 in two steps: warp w holds the rows of the residues
+// (w, R2 − w) modulo R2 (warp 0: 0 and R2/2), which the real transform's pairs (q, H − q) close over,
+// so that Z is formed in registers from loads that are all in flight at once; R1-point transforms,
+// twiddles, one exchange through shared memory, R2-point transforms. The 32 columns' rden rows stay in
+// shared memory while the block walks a run of items of one j. Each item's largest value is reduced
+// over the block first and its index looked for only in the warps that hold it. A slab of more than
+// 32 columns has several blocks: its candidate is a 64-bit key (the value, order-preserving; then the
+// lowest index), combined by atomicMax over zeroed scratch.
+// Bound by the loads' latency and issue together: U is read once, at 3.1 (H = 128) to 3.5 TB/s (H = 64)
+// of 6.5 measured; the shared-memory transform it takes over from (k_slab) ran at 0.2 TB/s, every
+// radix-2 stage a trip through shared memory between block barriers.
+struct SplitKey {
+  // float → unsigned, preserving the order (never 0 for a value a transform gives)
+  static __device__ __forceinline__ uint32_t ordered(float v) {
+    const uint32_t u = __float_as_uint(v);
+    return u ^ ((uint32_t)((int32_t)u >> 31) | 0x80000000u);
+  }
+  static __device__ __forceinline__ float value(uint32_t o) {
+    return __uint_as_float(o & 0x80000000u ? o ^ 0x80000000u : ~o);
+  }
+};
+
+template <int R1, int R2>
+struct SplitSmem {
+  static constexpr int H = R1 * R2, N = 2 * H;
+  static constexpr int RLD = N + 2;  // a row of rden, padded: 64-bit reads of 32 rows hit distinct banks
+  static constexpr size_t EX = (size_t)H * 32 * sizeof(float2);
+  static constexpr size_t RT = (size_t)32 * RLD * sizeof(float);
+  static constexpr size_t BYTES = EX + RT + (size_t)N * sizeof(float2);
+};
+
+template <int R1, int R2, int PER_SM>
+__global__ void __launch_bounds__(R2 * 16, PER_SM) k_slab_split(SlabArgs a, int chunk) {
+  using S = SplitSmem<R1, R2>;
+  constexpr int N = S::N, W = R2 / 2, G = R1 / W;  // G transforms of R2 points a warp
+  extern __shared__ __align__(16) uint8_t split_smem[];
+  float2* ex = (float2*)split_smem;                          // [R2][R1][32]
+  float* rt = (float*)(split_smem + S::EX);                  // [32][RLD]
+  float2* tws = (float2*)(split_smem + S::EX + S::RT);       // e^{−2πi t/N}
+  __shared__ float wmax[W];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int L = a.d.L, nc = a.d.nc, nb = a.d.nb;
+  const int nct = nc >> 5;
+  const int ct = blockIdx.x % nct;
+  const int j = (blockIdx.x / nct) % nb;
+  const int b0 = (blockIdx.x / (nct * nb)) * chunk;
+  const int b1 = min(a.n_items, b0 + chunk);
+  const int c = ct * 32 + lane;
+  for (int t = threadIdx.x; t < N; t += R2 * 16) tws[t] = __ldg(a.tw + t * (ZEB_TW_LEN / N));
+  const int ra = warp, rb = warp == 0 ? R2 / 2 : R2 - warp;
+  const uint32_t base = ((uint32_t)(j * nc + c)) * N;
+  int vol = -1;
+  for (int b = b0; b < b1; ++b) {
+    float2 xa[R1], xb[R1];
+    {
+      const float2* src = a.U + ((size_t)b * nb + j) * L * nc + c;
+#pragma unroll
+      for (int k = 0; k < R1; ++k) {
+        const int qa = ra + R2 * k, qb = rb + R2 * k;
+        xa[k] = qa < L ? __ldcs(src + (size_t)qa * nc) : make_float2(0.f, 0.f);
+        xb[k] = qb < L ? __ldcs(src + (size_t)qb * nc) : make_float2(0.f, 0.f);
+      }
+    }
+    if (b / a.rden_div != vol) {
+      // (the first item of the run, or of another rden volume; the barrier: the last reads of rt)
+      vol = b / a.rden_div;
+      __syncthreads();
+      const float* g = a.rden + (((size_t)vol * nb + j) * nc + (size_t)ct * 32) * N;
+      for (int e = threadIdx.x; e < 32 * N / 2; e += R2 * 16) {
+        const int row = e / (N / 2), p = e - row * (N / 2);
+        *(float2*)(rt + row * S::RLD + 2 * p) = __ldg((const float2*)g + e);
+      }
+      __syncthreads();
+    }
+    // Z_q = s + i t and Z_{H−q} = conj(s) + i conj(t), s = X_q + conj X_{H−q}, t = w_q (X_q − conj X_{H−q})
+    auto pair = [&](float2& xq, float2& xm, int q) {
+      const float2 w = tws[q];
+      const float2 sm = make_float2(xq.x + xm.x, xq.y - xm.y), df = make_float2(xq.x - xm.x, xq.y + xm.y);
+      const float2 t = make_float2(w.x * df.x - w.y * df.y, w.x * df.y + w.y * df.x);
+      xq = make_float2(sm.x - t.y, sm.y + t.x);
+      xm = make_float2(sm.x + t.y, t.x - sm.y);
+    };
+    if (warp == 0) {
+      // q = 0 alone (its own imaginary part dropped), q = H/2 with itself (2X)
+      xa[0] = make_float2(xa[0].x, xa[0].x);
+      xa[R1 / 2] = make_float2(2.f * xa[R1 / 2].x, 2.f * xa[R1 / 2].y);
+#pragma unroll
+      for (int k = 1; k < R1 / 2; ++k) pair(xa[k], xa[R1 - k], R2 * k);
+#pragma unroll
+      for (int k = 0; k < R1 / 2; ++k) pair(xb[k], xb[R1 - 1 - k], R2 / 2 + R2 * k);
+    } else {
+#pragma unroll
+      for (int k = 0; k < R1; ++k) pair(xa[k], xb[R1 - 1 - k], ra + R2 * k);
+    }
+    fft_reg<R1>(xa);
+    fft_reg<R1>(xb);
+#pragma unroll
+    for (int k = 0; k < R1; ++k) {
+      if (k > 0) {
+        xa[k] = cmulf(xa[k], tws[2 * ra * k]);
+        xb[k] = cmulf(xb[k], tws[(2 * rb * k) & (N - 1)]);
+      }
+      ex[(ra * R1 + k) * 32 + lane] = xa[k];
+      ex[(rb * R1 + k) * 32 + lane] = xb[k];
+    }
+    __syncthreads();
+    float2 z[G][R2];
+    float mx = -3.4e38f;
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      const int p1 = warp * G + g;
+#pragma unroll
+      for (int q2 = 0; q2 < R2; ++q2) z[g][q2] = ex[(q2 * R1 + p1) * 32 + lane];
+      fft_reg<R2>(z[g]);
+#pragma unroll
+      for (int p2 = 0; p2 < R2; ++p2) {
+        const float2 r = *(const float2*)(rt + lane * S::RLD + 2 * (p1 + R1 * p2));
+        z[g][p2].x *= r.x;
+        z[g][p2].y *= r.y;
+        mx = fmaxf(mx, fmaxf(z[g][p2].x, z[g][p2].y));
+      }
+    }
+    float wm = mx;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) wm = fmaxf(wm, __shfl_xor_sync(0xffffffffu, wm, o));
+    if (lane == 0) wmax[warp] = wm;
+    __syncthreads();
+    float bm = wmax[0];
+#pragma unroll
+    for (int w = 1; w < W; ++w) bm = fmaxf(bm, wmax[w]);
+    if (wm == bm) {  // (warp-uniform) this warp holds the block's largest value: its lowest index
+      uint32_t bi = 0xffffffffu;
+#pragma unroll
+      for (int g = 0; g < G; ++g)
+#pragma unroll
+        for (int p2 = 0; p2 < R2; ++p2) {
+          const uint32_t i0 = base + 2 * (warp * G + g + R1 * p2);
+          if (z[g][p2].x == bm) bi = min(bi, i0);
+          if (z[g][p2].y == bm) bi = min(bi, i0 + 1);
+        }
+      bi = __reduce_min_sync(0xffffffffu, bi);
+      if (lane == 0)
+        atomicMax((unsigned long long*)a.cand + (size_t)b * nb + j,
+                  ((unsigned long long)SplitKey::ordered(bm + 0.f) << 32) | (0xffffffffu - bi));
+    }
+  }
+}
+
 // V[j; m', c] of item b: U is already transformed along c (so3.wgsl:667-674)
 struct UReader32 {  // FP32, [item][j][m'][c]
   const float2* U;
@@ -356,6 +510,11 @@ __global__ void __launch_bounds__(64) k_peak_finish(SlabArgs a, R v_at, float* _
     for (int j = threadIdx.x; j < nb; j += 32) {
       float2 c = a.cand[(size_t)b * nb + j];
       uint32_t ci = __float_as_uint(c.y);
+      if (a.keyed) {  // (k_slab_split's; an untouched key is no candidate)
+        if ((__float_as_uint(c.x) | __float_as_uint(c.y)) == 0u) continue;
+        ci = ~__float_as_uint(c.x);
+        c.x = SplitKey::value(__float_as_uint(c.y));
+      }
       if (c.x > bv || (c.x == bv && ci < bi)) { bv = c.x; bi = ci; }
     }
 #pragma unroll
@@ -460,6 +619,26 @@ extern "C" size_t zeb_peaks_scratch_bytes(const zeb_so3_dims_t* d, int n_items) 
   return (size_t)n_items * d->nb * sizeof(float2);
 }
 
+// k_slab_split over every (item, j, 32 columns): runs of items long enough that staging a run's rden
+// rows (as many bytes as an item's U) costs a few per cent, short enough to leave the GPU several
+// waves of blocks
+template <int R1, int R2, int PER_SM>
+static int split_launch(SlabArgs& a, int sms, cudaStream_t st) {
+  using S = SplitSmem<R1, R2>;
+  const long long per_run = (long long)a.d.nb * (a.d.nc / 32);
+  const long long all = per_run * a.n_items, waves = 6LL * sms * PER_SM;
+  long long chunk = all / waves;
+  chunk = chunk < 1 ? 1 : chunk > 64 ? 64 : chunk;
+  const long long blocks = per_run * ((a.n_items + chunk - 1) / chunk);
+  ZEB_REQUIRE(blocks < (1LL << 31), ZEB_ESIZE, "correlate: too many slabs");
+  a.keyed = 1;
+  cudaError_t e = cudaMemsetAsync(a.cand, 0, (size_t)a.n_items * a.d.nb * sizeof(float2), st);
+  ZEB_REQUIRE(e == cudaSuccess, ZEB_ECUDA, "correlate slab (split): %s", cudaGetErrorString(e));
+  cudaFuncSetAttribute(k_slab_split<R1, R2, PER_SM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::BYTES);
+  k_slab_split<R1, R2, PER_SM><<<(unsigned)blocks, R2 * 16, S::BYTES, st>>>(a, (int)chunk);
+  return zeb_launch_check("correlate slab (split)");
+}
+
 static int slab_launch(const float* U, int n_items, const zeb_so3_dims_t* d, const float* tw, SlabArgs& a, bool vol,
                        cudaStream_t st) {
   a.U = (const float2*)U;
@@ -503,8 +682,13 @@ static int slab_launch(const float* U, int n_items, const zeb_so3_dims_t* d, con
     ZEB_SLAB_COLS(32, 32, 4, 4)
     ZEB_SLAB_COLS(64, 32, 4, 4)
     ZEB_SLAB_COLS(32, 64, 4, 3)
-    ZEB_SLAB_COLS(64, 64, 4, 3)
 #undef ZEB_SLAB_COLS
+    // Longer columns, and more columns than a warp's share of shared memory stages, take the block-wide
+    // split; measured on both sides of each line (items: before → split): L = 128, nc = 64 (256): 10.17
+    // → 0.70 ms; L = 80, nc = 128 (128): 9.47 → 0.59; L = 64, nc = 128 (1024): 19.7 → 1.23; L = 64, nc = 64
+    // (2048): 1.99 (k_slab_cols) → 1.23; but nc = 32 (4096): 1.10 against 1.25, and stays with k_slab_cols.
+    if (H == 128 && NC % 32 == 0) return split_launch<16, 8, 3>(a, sms, st);
+    if (H == 64 && NC % 32 == 0) return split_launch<8, 8, 4>(a, sms, st);
   }
   if (vol) {
     cudaFuncSetAttribute(k_slab<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
