@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(256) k_prep(PrepArgs a) {
     } else {
       const int s = a.bin, cp = a.cpad;
       const int hs = (h + s - 1) / s, ws = (w + s - 1) / s, wp = ws + 2 * cp, hp = hs + 2 * cp;
-      float2* box = (float2*)(a.scratch + (size_t)b * a.scratch_per + (a.use_smem ? 0 : hw));
+      float2* box = (float2*)(a.scratch + (size_t)b * a.scratch_per + (a.use_smem ? 0 : (hw + 1) & ~1));
       float2* rows = box + hs * ws;
       float2* cols = rows + hs * wp;
       float2* spread = cols + hp * wp;
@@ -411,7 +411,7 @@ static WideDims wide_dims(int h, int w, float sigma) {
 
 static long long scratch_floats(int h, int w, float sigma, int dynamic, bool smem) {
   long long per = 0;
-  if (!smem) per += (long long)h * w;  // the row-blurred image
+  if (!smem) per += ((long long)h * w + 1) & ~1LL;  // the row-blurred image, to an even count
   if (dynamic && sigma > 0.f) {
     WideDims d = wide_dims(h, w, sigma);
     if (d.bin >= 2) per += 2LL * (d.hs * d.ws + d.hs * d.wp + d.hp * d.wp + (long long)d.hp * w);
