@@ -46,32 +46,51 @@ __device__ __forceinline__ float2 wide_cell(int jr, int n, int s) {
   return make_float2(0.5f * (float)(lo + hi - 1), (float)(hi - lo));
 }
 
-// zero mean and unit norm under the mask (prep.wgsl:405-443), or the plain copy out
+// a thread's pixels i = threadIdx.x, + blockDim.x, … by row and column, without a division a pixel
+struct PixelWalk {
+  int i, r, c, dr, dc, w;
+  __device__ __forceinline__ explicit PixelWalk(int width) : i(threadIdx.x), w(width) {
+    r = i / w;
+    c = i - r * w;
+    dr = blockDim.x / w;
+    dc = blockDim.x - dr * w;
+  }
+  __device__ __forceinline__ void next() {
+    i += blockDim.x;
+    r += dr;
+    c += dc;
+    if (c >= w) {
+      c -= w;
+      ++r;
+    }
+  }
+};
+
+// zero mean and unit norm under the mask (prep.wgsl:405-443), or the plain copy out (img: the image in
+// shared memory, or out itself)
 __device__ void prep_finish(const PrepArgs& a, float* img, float* out, float* red) {
-  const int h = a.h, w = a.w, hw = h * w;
+  const int hw = a.h * a.w;
   if (!a.normalize) {
-    if (a.use_smem)
+    if (img != out)
       for (int i = threadIdx.x; i < hw; i += blockDim.x) out[i] = img[i];
     return;
   }
   float v2[2] = {0.f, 0.f};
-  for (int i = threadIdx.x; i < hw; i += blockDim.x) {
-    int r = i / w, c = i - r * w;
-    float dr = (float)r - a.mask[0], dc = (float)c - a.mask[1];
+  for (PixelWalk p(a.w); p.i < hw; p.next()) {
+    float dr = (float)p.r - a.mask[0], dc = (float)p.c - a.mask[1];
     if (zeb_in_circle(dr, dc, a.mask[2])) {
-      v2[0] += img[i];
+      v2[0] += img[p.i];
       v2[1] += 1.f;
     }
   }
   block_sums<2>(v2, red);
   const float mean = v2[0] / fmaxf(v2[1], 1.f);
   float ss[1] = {0.f};
-  for (int i = threadIdx.x; i < hw; i += blockDim.x) {
-    int r = i / w, c = i - r * w;
-    float dr = (float)r - a.mask[0], dc = (float)c - a.mask[1];
+  for (PixelWalk p(a.w); p.i < hw; p.next()) {
+    float dr = (float)p.r - a.mask[0], dc = (float)p.c - a.mask[1];
     float v = 0.f;
-    if (zeb_in_circle(dr, dc, a.mask[2])) v = img[i] - mean;
-    img[i] = v;
+    if (zeb_in_circle(dr, dc, a.mask[2])) v = img[p.i] - mean;
+    img[p.i] = v;
     ss[0] += v * v;
   }
   block_sums<1>(ss, red);
@@ -145,6 +164,24 @@ __device__ __forceinline__ float prep_pixel(const PrepArgs& a, int b, int i) {
   }
   if (a.static_bg) v -= __ldg(a.static_bg + i);
   return v;
+}
+
+// every pixel of pattern b, put(pixel walk, value) in the block's order; the usual case (nothing reduced,
+// a static background) without a branch a pixel
+template <typename T, typename Put>
+__device__ __forceinline__ void unpack_as(const PrepArgs& a, int b, Put put) {
+  const T* raw = (const T*)a.raw + (size_t)b * a.h * a.w;
+  for (PixelWalk p(a.w); p.i < a.h * a.w; p.next()) put(p, (float)raw[p.i] - __ldg(a.static_bg + p.i));
+}
+template <typename Put>
+__device__ __forceinline__ void unpack(const PrepArgs& a, int b, Put put) {
+  if (a.factor == 1.0 && a.static_bg) {
+    if (a.pixel == 0) unpack_as<uint8_t>(a, b, put);
+    else if (a.pixel == 1) unpack_as<uint16_t>(a, b, put);
+    else unpack_as<float>(a, b, put);
+  } else {
+    for (PixelWalk p(a.w); p.i < a.h * a.w; p.next()) put(p, prep_pixel(a, b, p.i));
+  }
 }
 
 __global__ void __launch_bounds__(256) k_prep(PrepArgs a) {
@@ -288,6 +325,8 @@ __global__ void __launch_bounds__(256) k_prep(PrepArgs a) {
 // load serves several FMAs (the taps beyond 2R are zeros, adding exact zeros).  Each output sums
 // its taps in increasing order with fmaf, the order of k_prep, so the results are the same bits;
 // the taps inside the image are summed once per column and per row for the edge renormalization.
+// Bound by instruction issue: steps wholly in the padding are skipped, and no loop over the pixels
+// divides (16 384 u16 patterns of 60 × 60: 1187 → 949 µs).
 constexpr int PD_OUT = 16;  // outputs a thread takes along the blur
 constexpr int PD_TB = 8;    // taps a step
 
@@ -317,10 +356,7 @@ __global__ void __launch_bounds__(256) k_prep_direct(PrepArgs a) {
   for (int i = threadIdx.x; i < R * w; i += blockDim.x) Q[i] = 0.f;
   for (int i = threadIdx.x; i < (qr - R - h) * w; i += blockDim.x) Q[(R + h) * w + i] = 0.f;
   __syncthreads();
-  for (int i = threadIdx.x; i < hw; i += blockDim.x) {
-    const int r = i / w, c = i - r * w;
-    P[r * pw + R + c] = prep_pixel(a, b, i);
-  }
+  unpack(a, b, [&](const PixelWalk& p, float v) { P[p.r * pw + R + p.c] = v; });
   for (int k = threadIdx.x; k < w + h; k += blockDim.x) {
     const int n = k < w ? w : h, c = k < w ? k : k - w;
     float g = 0.f;
@@ -337,7 +373,9 @@ __global__ void __launch_bounds__(256) k_prep_direct(PrepArgs a) {
     float acc[PD_OUT];
 #pragma unroll
     for (int k = 0; k < PD_OUT; ++k) acc[k] = 0.f;
-    for (int d0 = 0; d0 < nblk * PD_TB; d0 += PD_TB) {
+    // only the steps that reach the image (the others add exact zeros)
+    const int first = c0 + PD_OUT + PD_TB - 2 < R ? (R - c0 - PD_OUT - PD_TB + 2 + PD_TB - 1) & ~(PD_TB - 1) : 0;
+    for (int d0 = first; d0 < nblk * PD_TB && c0 + d0 < R + w; d0 += PD_TB) {
       float x[PD_OUT + PD_TB - 1];
       const float4 ta = *reinterpret_cast<const float4*>(taps + d0);
       const float4 tb = *reinterpret_cast<const float4*>(taps + d0 + 4);
@@ -363,7 +401,8 @@ __global__ void __launch_bounds__(256) k_prep_direct(PrepArgs a) {
     float acc[PD_OUT];
 #pragma unroll
     for (int k = 0; k < PD_OUT; ++k) acc[k] = 0.f;
-    for (int d0 = 0; d0 < nblk * PD_TB; d0 += PD_TB) {
+    const int first = r0 + PD_OUT + PD_TB - 2 < R ? (R - r0 - PD_OUT - PD_TB + 2 + PD_TB - 1) & ~(PD_TB - 1) : 0;
+    for (int d0 = first; d0 < nblk * PD_TB && r0 + d0 < R + h; d0 += PD_TB) {
       float x[PD_OUT + PD_TB - 1];
       const float4 ta = *reinterpret_cast<const float4*>(taps + d0);
       const float4 tb = *reinterpret_cast<const float4*>(taps + d0 + 4);
@@ -386,12 +425,244 @@ __global__ void __launch_bounds__(256) k_prep_direct(PrepArgs a) {
   }
   __syncthreads();
   // the combined image, contiguous, where Q was
-  for (int i = threadIdx.x; i < hw; i += blockDim.x) {
-    const int r = i / w, c = i - r * w;
-    Q[i] = P[r * pw + R + c];
-  }
+  for (PixelWalk p(w); p.i < hw; p.next()) Q[p.i] = P[p.r * pw + R + p.c];
   __syncthreads();
   prep_finish(a, Q, a.out + base, red);
+}
+
+// The wide blur with what does not depend on the pattern made once a call (k_wide_tables): the coarse
+// Gaussian's weights, the spread's weights and the weights' own sum at every pixel. k_prep forms all of
+// them again for each pattern, two exponentials a tap and pixel, and passes its partial sums through
+// global memory; here a block keeps the partial sums (and the image, where two blocks fit an SM) in
+// shared memory, and the two coarse passes, most of the products, run in register tiles. Every sum runs
+// in k_prep's order over the same weights: the results are the same bits. Bound by instruction issue.
+// u16 patterns with their background off and normalized: 3072 of 96 × 96 1378 → 509 µs, 4096 of 120 × 120
+// 2350 → 1173, 2048 of 160 × 160 1468 → 980, 5 of 160 × 80 158 → 116.
+struct WideTables {
+  float *den;       // [h][w]: the weights' sum
+  float *wx, *wy;   // [ws4][wp], [hs][hp8]: the coarse Gaussian, box j to coarse cell t; 0 out of reach
+  float *sx, *sy;   // [kWideQ][w], [kWideQ][h]: a coarse cell's spread to a pixel
+};
+constexpr int kWideCpad = 3, kWideQ = 2 * kWideCpad + 1;
+constexpr int kWideRowTile = 6, kWideColTile = 8;  // box lines, coarse cells down the columns, a thread
+
+struct WideShape {
+  int hs, ws, hp, wp, ws4, hp8;
+  __host__ __device__ WideShape(int h, int w, int s) {
+    hs = (h + s - 1) / s;
+    ws = (w + s - 1) / s;
+    hp = hs + 2 * kWideCpad;
+    wp = ws + 2 * kWideCpad;
+    ws4 = (ws + 3) & ~3;
+    hp8 = (hp + 7) & ~7;
+  }
+  __host__ __device__ int lines() const { return (hs + kWideRowTile - 1) / kWideRowTile * kWideRowTile; }
+  // the tables in floats; den first, wy on a 16-byte boundary
+  __host__ __device__ long long table_floats(int h, int w) const {
+    return (((long long)h * w + (long long)ws4 * wp + 3) & ~3LL) + (long long)hs * hp8 + kWideQ * (long long)(h + w);
+  }
+  __host__ __device__ WideTables tables(float* t, int h, int w) const {
+    WideTables o;
+    o.den = t;
+    o.wx = t + (long long)h * w;
+    o.wy = t + (((long long)h * w + (long long)ws4 * wp + 3) & ~3LL);
+    o.sx = o.wy + (long long)hs * hp8;
+    o.sy = o.sx + kWideQ * (long long)w;
+    return o;
+  }
+  // shared memory of k_prep_wide without the image, in floats: box sums and their rows, or the spread; then
+  // the coarse image
+  __host__ __device__ int first(int w) const {
+    const int coarse = lines() * (ws4 + wp);
+    return ((hp * w > coarse ? hp * w : coarse) + 3) & ~3;
+  }
+  __host__ __device__ int part(int w) const { return first(w) + hp8 * wp; }
+};
+
+// weight of box j for coarse cell t of an axis of n pixels in `cells` boxes (0 out of reach)
+__device__ __forceinline__ float wide_coarse(const PrepArgs& a, int t, int j, int n, int cells) {
+  const int s = a.bin;
+  const float reach = (float)a.wradius;
+  const float c = wide_cell(t - kWideCpad, n, s).x;
+  const int j0 = max((int)floorf((c - reach) / (float)s), 0);
+  const int j1 = min((int)floorf((c + reach) / (float)s), cells - 1);
+  if (j < j0 || j > j1) return 0.f;
+  const float d = wide_cell(j, n, s).x - c;
+  return expf(-d * d * a.kx);
+}
+// weight of coarse cell x / s + q − cpad for pixel x of an axis of n pixels
+__device__ __forceinline__ float wide_spread(const PrepArgs& a, int x, int q, int n) {
+  const float2 cw = wide_cell(x / a.bin + q - kWideCpad, n, a.bin);
+  const float d = (float)x - cw.x;
+  return cw.y * expf(-d * d * a.kz);
+}
+
+// A block makes the weights' sum of one pixel row; the first block writes the other tables too. The box
+// lines of a pattern hold s rows each but the last, so two lines' row sums stand for all.
+__global__ void __launch_bounds__(256) k_wide_tables(PrepArgs a, float* out) {
+  extern __shared__ float sm[];
+  const int h = a.h, w = a.w, s = a.bin, y = blockIdx.x, own = y / s;
+  const WideShape d(h, w, s);
+  const WideTables T = d.tables(out, h, w);
+  float* ex = sm;                       // [ws][wp]
+  float* ey = ex + d.ws * d.wp;         // [kWideQ][hs]: the weights of the row's coarse cells
+  float* line = ey + kWideQ * d.hs;     // [2][wp]: the row sums of a whole line and of the last
+  float* cols = line + 2 * d.wp;        // [kWideQ][wp]
+  for (int t = threadIdx.x; t < d.ws * d.wp; t += blockDim.x) ex[t] = wide_coarse(a, t % d.wp, t / d.wp, w, d.ws);
+  for (int t = threadIdx.x; t < kWideQ * d.hs; t += blockDim.x) ey[t] = wide_coarse(a, own + t / d.hs, t % d.hs, h, d.hs);
+  if (y == 0) {
+    for (int t = threadIdx.x; t < d.ws4 * d.wp; t += blockDim.x)
+      T.wx[t] = t < d.ws * d.wp ? wide_coarse(a, t % d.wp, t / d.wp, w, d.ws) : 0.f;
+    for (int t = threadIdx.x; t < d.hs * d.hp8; t += blockDim.x) {
+      const int tr = t % d.hp8;
+      T.wy[t] = tr < d.hp ? wide_coarse(a, tr, t / d.hp8, h, d.hs) : 0.f;
+    }
+    for (int t = threadIdx.x; t < kWideQ * w; t += blockDim.x) T.sx[t] = wide_spread(a, t % w, t / w, w);
+    for (int t = threadIdx.x; t < kWideQ * h; t += blockDim.x) T.sy[t] = wide_spread(a, t % h, t / h, h);
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < 2 * d.wp; t += blockDim.x) {
+    const int last = t / d.wp, tc = t - last * d.wp;
+    const int rows = last ? h - (d.hs - 1) * s : s;
+    float acc = 0.f;
+    for (int j = 0; j < d.ws; ++j) {
+      const float e = ex[j * d.wp + tc];
+      if (e != 0.f) acc = fmaf(e, (float)(rows * (min((j + 1) * s, w) - j * s)), acc);
+    }
+    line[t] = acc;
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < kWideQ * d.wp; t += blockDim.x) {
+    const int q = t / d.wp, col = t - q * d.wp;
+    float acc = 0.f;
+    for (int i = 0; i < d.hs; ++i) {
+      const float e = ey[q * d.hs + i];
+      if (e != 0.f) acc = fmaf(e, line[(i == d.hs - 1 ? d.wp : 0) + col], acc);
+    }
+    cols[t] = acc;
+  }
+  __syncthreads();
+  for (int x = threadIdx.x; x < w; x += blockDim.x) {
+    float e[kWideQ], acc = 0.f;
+#pragma unroll
+    for (int k = 0; k < kWideQ; ++k) e[k] = wide_spread(a, x, k, w);
+#pragma unroll
+    for (int q = 0; q < kWideQ; ++q) {
+      float sp = 0.f;
+#pragma unroll
+      for (int k = 0; k < kWideQ; ++k) sp = fmaf(e[k], cols[q * d.wp + x / s + k], sp);
+      acc = fmaf(wide_spread(a, y, q, h), sp, acc);
+    }
+    T.den[(size_t)y * w + x] = acc;
+  }
+}
+
+__global__ void __launch_bounds__(256) k_prep_wide(PrepArgs a, float* tables, int img_smem) {
+  extern __shared__ __align__(16) float sm[];
+  __shared__ float red[2 * 8];
+  const int h = a.h, w = a.w, hw = h * w, s = a.bin;
+  const WideShape d(h, w, s);
+  const WideTables T = d.tables(tables, h, w);
+  const size_t base = (size_t)blockIdx.x * hw;
+  float* spread = sm;                     // [hp][w]; before it:
+  float* box = sm;                        // [lines][ws4]
+  float* rows = sm + d.lines() * d.ws4;   // [lines][wp]
+  float* cols = sm + d.first(w);          // [hp8][wp]
+  float* img = img_smem ? sm + d.part(w) : a.out + base;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  unpack(a, blockIdx.x, [&](const PixelWalk& p, float v) { img[p.i] = v; });
+  __syncthreads();
+  for (int i = warp; i < d.lines(); i += nw) {
+    const int r1 = min((i + 1) * s, h);
+    for (int j = lane; j < d.ws4; j += 32) {
+      const int c1 = min((j + 1) * s, w);
+      float acc = 0.f;
+      for (int r = i * s; r < r1; ++r)
+        for (int c = j * s; c < c1; ++c) acc += img[r * w + c];
+      box[i * d.ws4 + j] = acc;
+    }
+  }
+  __syncthreads();
+  // the coarse Gaussian along the rows: a thread takes six lines of one coarse column
+  const int tx = (d.wp + 31) / 32;
+  for (int t = warp; t < d.lines() / kWideRowTile * tx; t += nw) {
+    const int i0 = t / tx * kWideRowTile, tc = (t % tx) * 32 + lane;
+    float acc[kWideRowTile];
+#pragma unroll
+    for (int k = 0; k < kWideRowTile; ++k) acc[k] = 0.f;
+    const float* wx = T.wx + min(tc, d.wp - 1);
+    for (int j = 0; j < d.ws4; j += 4) {
+      float e[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) e[q] = __ldg(wx + (j + q) * d.wp);
+#pragma unroll
+      for (int k = 0; k < kWideRowTile; ++k) {
+        const float4 v = *(const float4*)(box + (i0 + k) * d.ws4 + j);
+        if (e[0] != 0.f) acc[k] = fmaf(e[0], v.x, acc[k]);
+        if (e[1] != 0.f) acc[k] = fmaf(e[1], v.y, acc[k]);
+        if (e[2] != 0.f) acc[k] = fmaf(e[2], v.z, acc[k]);
+        if (e[3] != 0.f) acc[k] = fmaf(e[3], v.w, acc[k]);
+      }
+    }
+    if (tc < d.wp)
+#pragma unroll
+      for (int k = 0; k < kWideRowTile; ++k) rows[(i0 + k) * d.wp + tc] = acc[k];
+  }
+  __syncthreads();
+  // and along the columns: eight coarse cells of one column
+  for (int t = warp; t < d.hp8 / kWideColTile * tx; t += nw) {
+    const int tr0 = t / tx * kWideColTile, col = (t % tx) * 32 + lane;
+    float acc[kWideColTile];
+#pragma unroll
+    for (int k = 0; k < kWideColTile; ++k) acc[k] = 0.f;
+    const float* src = rows + min(col, d.wp - 1);
+#pragma unroll 2
+    for (int i = 0; i < d.hs; ++i) {
+      const float4 ea = __ldg((const float4*)(T.wy + i * d.hp8 + tr0)), eb = __ldg((const float4*)(T.wy + i * d.hp8 + tr0 + 4));
+      const float v = src[i * d.wp];
+      if (ea.x != 0.f) acc[0] = fmaf(ea.x, v, acc[0]);
+      if (ea.y != 0.f) acc[1] = fmaf(ea.y, v, acc[1]);
+      if (ea.z != 0.f) acc[2] = fmaf(ea.z, v, acc[2]);
+      if (ea.w != 0.f) acc[3] = fmaf(ea.w, v, acc[3]);
+      if (eb.x != 0.f) acc[4] = fmaf(eb.x, v, acc[4]);
+      if (eb.y != 0.f) acc[5] = fmaf(eb.y, v, acc[5]);
+      if (eb.z != 0.f) acc[6] = fmaf(eb.z, v, acc[6]);
+      if (eb.w != 0.f) acc[7] = fmaf(eb.w, v, acc[7]);
+    }
+    if (col < d.wp)
+#pragma unroll
+      for (int k = 0; k < kWideColTile; ++k) cols[(tr0 + k) * d.wp + col] = acc[k];
+  }
+  __syncthreads();
+  // the coarse cells spread to the pixels, along the rows and then down the columns
+  for (int x = lane; x < w; x += 32) {
+    float e[kWideQ];
+#pragma unroll
+    for (int q = 0; q < kWideQ; ++q) e[q] = __ldg(T.sx + q * w + x);
+    const float* src = cols + x / s;
+    for (int tr = warp; tr < d.hp; tr += nw) {
+      float acc = 0.f;
+#pragma unroll
+      for (int q = 0; q < kWideQ; ++q) acc = fmaf(e[q], src[tr * d.wp + q], acc);
+      spread[tr * w + x] = acc;
+    }
+  }
+  __syncthreads();
+  for (int y = warp; y < h; y += nw) {
+    float e[kWideQ];
+#pragma unroll
+    for (int q = 0; q < kWideQ; ++q) e[q] = __ldg(T.sy + q * h + y);
+    const float* src = spread + y / s * w;
+    for (int x = lane; x < w; x += 32) {
+      float acc = 0.f;
+#pragma unroll
+      for (int q = 0; q < kWideQ; ++q) acc = fmaf(e[q], src[q * w + x], acc);
+      const float bgv = acc / __ldg(T.den + y * w + x);
+      img[y * w + x] = with_background(a.dynamic, img[y * w + x], bgv);
+    }
+  }
+  __syncthreads();
+  prep_finish(a, img, a.out + base, red);
 }
 
 struct WideDims {
@@ -476,6 +747,24 @@ static int prep_launch(const void* raw, int pixel, int n, int src_h, int src_w, 
       cudaFuncSetAttribute(k_prep_direct, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsm);
       k_prep_direct<<<n, 256, dsm, (cudaStream_t)stream>>>(a);
       return zeb_launch_check("prep (direct blur)");
+    }
+  }
+  if (a.dynamic && a.bin >= 2) {
+    const WideShape d(h, w, a.bin);
+    const size_t part = (size_t)d.part(w) * 4, whole = part + (size_t)h * w * 4;
+    // the image in shared memory while two blocks fit an SM, else where the result goes (L2 holds it)
+    const bool in = whole <= 113 * 1024;
+    const size_t wsm = in ? whole : part, tsm = (size_t)(d.ws * d.wp + kWideQ * (d.hs + d.wp) + 2 * d.wp) * 4;
+    // the tables take the place of the partial sums in the caller's scratch, whose size stays what it was:
+    // one pattern of a large detector may not have the room
+    if (d.table_floats(h, w) <= a.scratch_per * n && wsm <= 200 * 1024 && tsm <= 200 * 1024 && ((uintptr_t)scratch & 15) == 0) {
+      if (tsm > 48 * 1024) cudaFuncSetAttribute(k_wide_tables, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm);
+      k_wide_tables<<<h, 256, tsm, (cudaStream_t)stream>>>(a, a.scratch);
+      int rc = zeb_launch_check("prep (wide blur tables)");
+      if (rc) return rc;
+      if (wsm > 48 * 1024) cudaFuncSetAttribute(k_prep_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wsm);
+      k_prep_wide<<<n, 256, wsm, (cudaStream_t)stream>>>(a, a.scratch, in ? 1 : 0);
+      return zeb_launch_check("prep (wide blur)");
     }
   }
   size_t smem = a.use_smem ? 2 * (size_t)h * w * 4 : 0;
