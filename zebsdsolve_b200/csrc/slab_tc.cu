@@ -22,9 +22,16 @@
 //
 // One persistent CTA per SM: warp 0 issues the tensor loads (a ring of ST_STAGES tiles) and the
 // bulk copies of each tile's row of rden (a ring of ST_RSLOTS), warp 1 the MMAs into ST_ACC
-// accumulators of n columns, warps 2-9 drain them (two warps per TMEM lane quadrant, each half of
-// the n columns).  Every wait is bounded: on a timeout the CTA records the
+// accumulators of n columns, the others drain them (in groups of eight: two warps per TMEM lane
+// quadrant, each half of the n columns).  Every wait is bounded: on a timeout the CTA records the
 // failure, waits (bounded) for what it issued, frees its TMEM and returns.
+//
+// What bounds it: n = 128 the MMAs (a tile is 8 K-steps of 128 × 128 against 64 KB of U, and the
+// issue of a tile follows the last one's; with one K-step of the eight 0.70 → 0.55 ms at 6144 items,
+// L = 64, nc = 32).  For n <= 64 a tile is a quarter of that or less, and the epilogue's time on it is
+// mostly latency (the wait, the tensor-memory load, the chain of maxima): a second group of eight
+// warps takes every other tile, 6144 items of L = 32 0.195 → 0.148 ms, 300 0.098 → 0.093; at
+// n = 128 the second group only adds its barriers (0.695 → 0.701), so one stays there.
 #include <cuda.h>
 #include <cuda_fp16.h>
 #include <cudaTypedefs.h>
@@ -38,8 +45,7 @@ namespace zeb {
 
 constexpr int ST_BM = 128;                  // items per tile (MMA M)
 constexpr int ST_STAGES = 4;                // tiles of U in flight
-constexpr int ST_EPI = 8;                   // epilogue warps
-constexpr int ST_THREADS = 64 + 32 * ST_EPI;
+constexpr int ST_GRP = 8;                   // epilogue warps a group
 constexpr int ST_HALF_BYTES = 16384;        // one 64-item half of a tile: 2L rows of 128 B (L <= 64)
 
 struct SlabTcArgs {
@@ -59,8 +65,8 @@ struct SlabTcShared {
   uint8_t f[2][16384];                        // F: n rows × 2L FP16, K-major, in 64-wide K blocks
   uint8_t a[ST_STAGES][2][ST_HALF_BYTES];     // tiles of U: [half][κ][64 items]
   float rden[ST_RSLOTS][128];                 // each tile's row rden[j][c][0 … n)
-  float bestv[2][ST_BM];                      // the second half's best, handed to the first
-  uint32_t besti[2][ST_BM];
+  float bestv[2][3][ST_BM];                   // the other halves' and groups' bests, handed to the first
+  uint32_t besti[2][3][ST_BM];
   uint64_t full[ST_STAGES], empty[ST_STAGES], acc_full[ST_ACC], acc_empty[ST_ACC], rfull[ST_RSLOTS],
       rempty[ST_RSLOTS], mma_done, never;
   uint32_t tmem;
@@ -82,7 +88,9 @@ __device__ void build_dft(uint8_t (*f)[16384], int n, int L) {
   }
 }
 
-__global__ void __launch_bounds__(ST_THREADS, 1) k_slab_tc(SlabTcArgs a, const __grid_constant__ CUtensorMap umap) {
+// GROUPS groups of epilogue warps take the tiles in turn; a thread holds COLS >= n/2 columns of a tile
+template <int GROUPS, int COLS>
+__global__ void __launch_bounds__(64 + 32 * ST_GRP * GROUPS, 1) k_slab_tc(SlabTcArgs a, const __grid_constant__ CUtensorMap umap) {
   extern __shared__ __align__(1024) uint8_t st_smem_raw[];
   SlabTcShared& s = *reinterpret_cast<SlabTcShared*>((void*)(((uintptr_t)st_smem_raw + 1023) & ~(uintptr_t)1023));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -98,11 +106,11 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_slab_tc(SlabTcArgs a, const _
     }
     for (int i = 0; i < ST_ACC; ++i) {
       mbar_init(&s.acc_full[i], 1);
-      mbar_init(&s.acc_empty[i], ST_EPI);
+      mbar_init(&s.acc_empty[i], ST_GRP);
     }
     for (int i = 0; i < ST_RSLOTS; ++i) {
       mbar_init(&s.rfull[i], 1);
-      mbar_init(&s.rempty[i], ST_EPI);
+      mbar_init(&s.rempty[i], ST_GRP);
     }
     mbar_init(&s.mma_done, 1);
     mbar_init(&s.never, 1);  // nothing arrives: the failure test's wait
@@ -192,13 +200,14 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_slab_tc(SlabTcArgs a, const _
       if (!mbar_wait(&s.mma_done, 0, kDrainNs)) atomicOr(a.status, 8);
     }
   } else {
-    // epilogue: warp w reads TMEM lanes 32·(w mod 4) …; warps w and w + 4 take the two halves of
-    // the n columns. Thread = one item (row of the tile) × half the a values of each tile. Each
-    // warp follows the accumulators on its own (the MMAs run up to ST_ACC tiles ahead); the eight
-    // meet once per item, where the halves' bests merge.
+    // epilogue: warp w reads TMEM lanes 32·(w mod 4) …; a group's warps w and w + 4 take the two halves
+    // of the n columns, the groups the tiles in turn. Thread = one item (row of the tile) × half the a
+    // values of each of its tiles. Each warp follows the accumulators on its own (the MMAs run up to
+    // ST_ACC tiles ahead); they all meet once per work item, where the bests merge.
     const int ew = warp & 3;
     const int row = ew * 32 + lane;
-    const int half = (warp - 2) >> 2;
+    const int half = ((warp - 2) >> 2) & 1, grp = (warp - 2) >> 3;
+    const int slot = grp * 2 + half - 1;  // (−1: the warps the bests are handed to)
     const int hn = n >> 1;  // columns per half: 16, 32 or 64
     const uint32_t lanes = (uint32_t)(ew * 32) << 16;
     const float rsc = a.rscale;
@@ -210,6 +219,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_slab_tc(SlabTcArgs a, const _
       const long long item = blockIdx.x + mi * gridDim.x;
       const int j = (int)(item / a.ptiles), pt = (int)(item - (long long)j * a.ptiles);
       for (int c = 0; c < nc && ok; ++c, ++t) {
+        if (GROUPS > 1 && (int)(t % GROUPS) != grp) continue;
         const int acc = (int)(t % ST_ACC);
         const int rs = (int)(t % ST_RSLOTS);
         // lane 0 waits (try_wait suspends it in hardware until the phase completes); the warp follows
@@ -225,9 +235,9 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_slab_tc(SlabTcArgs a, const _
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t c0 = tmem + lanes + (uint32_t)(acc * 128 + half * hn);
-        uint32_t v[64];
+        uint32_t v[COLS];
         TMEM_LD32(c0, v);
-        if (hn > 32) TMEM_LD32(c0 + 32, (v + 32));
+        if (COLS > 32) TMEM_LD32(c0 + 32, (v + 32));
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
@@ -235,9 +245,9 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_slab_tc(SlabTcArgs a, const _
         // the values s·C·rden (s a power of two: the order, and every product's rounding, are those
         // of C·rden; the candidate is scaled by 1/s once, exactly); their largest by a tree
         const float* rrow = s.rden[rs] + half * hn;
-        float x[64];
+        float x[COLS];
 #pragma unroll
-        for (int q = 0; q < 16; ++q) {
+        for (int q = 0; q < COLS / 4; ++q) {
           if (4 * q < hn) {
             const float4 r = *reinterpret_cast<const float4*>(rrow + 4 * q);
             x[4 * q + 0] = __uint_as_float(v[4 * q + 0]) * r.x;
@@ -255,32 +265,35 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_slab_tc(SlabTcArgs a, const _
         for (int k = 0; k < 4; ++k) {
           float m = x[k];
 #pragma unroll
-          for (int q = 1; q < 16; ++q) m = fmaxf(m, x[4 * q + k]);
+          for (int q = 1; q < COLS / 4; ++q) m = fmaxf(m, x[4 * q + k]);
           m4[k] = m;
         }
         const float m = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
         if (m > bv) {  // a new best: its first position in the tile (indices grow along the tile)
           int kk = 0;
 #pragma unroll
-          for (int k = 63; k >= 0; --k)
+          for (int k = COLS - 1; k >= 0; --k)
             if (x[k] == m) kk = k;
           bv = m;
           bi = (uint32_t)(j * nc + c) * (uint32_t)n + (uint32_t)(half * hn + kk);
         }
       }
-      // the item's end: the eight warps agree on the outcome, and the second half's best joins the
-      // first's (lower index on equal values)
+      // the work item's end: the warps agree on the outcome, and the other halves' and groups' bests
+      // join the first's (lower index on equal values)
       const int par = (int)(mi & 1);
-      if (half == 1) {
-        s.bestv[par][row] = bv;
-        s.besti[par][row] = bi;
+      if (slot >= 0) {
+        s.bestv[par][slot][row] = bv;
+        s.besti[par][slot][row] = bi;
       }
-      ok = bar_and(2, 32 * ST_EPI, ok);
+      ok = bar_and(2, 32 * ST_GRP * GROUPS, ok);
       if (!ok) break;
-      if (half == 0) {
-        const float ov = s.bestv[par][row];
-        const uint32_t oi = s.besti[par][row];
-        if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
+      if (slot < 0) {
+#pragma unroll
+        for (int k = 0; k < 2 * GROUPS - 1; ++k) {
+          const float ov = s.bestv[par][k][row];
+          const uint32_t oi = s.besti[par][k][row];
+          if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
+        }
         const int p = pt * ST_BM + row;
         if (p < a.n_items) a.cand[(size_t)p * nb + j] = make_float2(bv * rsc, __uint_as_float(bi));
       }
@@ -355,13 +368,16 @@ extern "C" int zeb_correlate_peaks_h(const void* U16, int n_items, const zeb_so3
   a.limit = a.stall > 0 ? a.stall : kWaitNs;
   cudaStream_t st = (cudaStream_t)stream;
   const size_t smem = sizeof(SlabTcShared) + 1024;
-  cudaFuncSetAttribute(k_slab_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const long long items = (long long)a.ptiles * d->nb;
   const int grid = (int)std::min<long long>(items, sms);
-  k_slab_tc<<<grid, ST_THREADS, smem, st>>>(a, umap);
+  // (each group's epilogue threads, and the columns of their half of a tile)
+  const int groups = d->n <= 64 ? 2 : 1;
+  auto kernel = groups == 2 ? k_slab_tc<2, 32> : k_slab_tc<1, 64>;
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  kernel<<<grid, 64 + 32 * ST_GRP * groups, smem, st>>>(a, umap);
   int rc = zeb_launch_check("correlate slab (tensor cores)");
   if (rc) return rc;
   return zeb_peak_finish_h(U16, n_items, d, scale, rden, (const float2*)scratch, peaks, stream);

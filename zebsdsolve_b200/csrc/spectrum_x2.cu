@@ -84,39 +84,40 @@ __global__ void k_x2_pack_master(const double2* __restrict__ Y, int L, int ncols
   *(uint4*)(p + X2_BLOCK) = pack8(hi);
 }
 
-// The patterns' blocks, [order][pattern tile][K-block][hi, lo]
-__global__ void k_x2_pack_patterns(const float2* __restrict__ alm, int n_items, int n_pairs, int L, int ptiles,
-                                   uint8_t* __restrict__ B) {
-  const int mp = blockIdx.y;
-  __shared__ long long first;
-  if (threadIdx.x == 0) first = x2_blocks_before(L, mp) * ptiles;
-  __syncthreads();
+// The patterns' blocks, [order][pattern tile][K-block][hi, lo]: a block per (K-block, pattern tile, order;
+// `most` K-blocks or fewer an order), a thread per 16-byte chunk (four degrees' re and im) of four rows
+__global__ void __launch_bounds__(256) k_x2_pack_patterns(const float2* __restrict__ alm, int n_items, int n_pairs, int L,
+                                                          int ptiles, int most, uint8_t* __restrict__ B) {
+  const int ptile = blockIdx.x / most, kblock = blockIdx.x - ptile * most, mp = blockIdx.y;
   const int kb = x2_kblocks(L, mp);
-  const long long chunks = (long long)ptiles * kb * 128 * 8;
-  const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= chunks) return;
-  const int c16 = (int)(e & 7), row = (int)((e >> 3) & 127);
-  const long long blk = e >> 10;
-  const int kblock = (int)(blk % kb);
-  const int b = (int)(blk / kb) * 128 + row;
+  if (kblock >= kb) return;
+  int before = 0;  // the blocks of the lower orders: a lane sums every 32nd of them
+  for (int q = threadIdx.x & 31; q < mp; q += 32) before += x2_kblocks(L, q);
+  before = __reduce_add_sync(0xffffffffu, before);
+  uint8_t* blk = B + ((size_t)before * ptiles + (size_t)ptile * kb + kblock) * 2 * X2_BLOCK;
   const int p0 = mp * L - (mp * (mp - 1)) / 2;
-  uint16_t hi[8], lo[8];
+  const int c16 = threadIdx.x & 7;
 #pragma unroll
-  for (int i = 0; i < 8; i += 2) {
-    const int l = L - 1 - ((kblock * X2_KB + c16 * 8 + i) >> 1);
-    float2 g = make_float2(0.f, 0.f);
-    if (l >= mp && b < n_items) g = __ldg(alm + (size_t)b * n_pairs + p0 + l - mp);
-    const float v[2] = {g.x * X2_PATTERN_SCALE, g.y * X2_PATTERN_SCALE};
+  for (int it = 0; it < 4; ++it) {
+    const int row = (threadIdx.x >> 3) + 32 * it, b = ptile * 128 + row;
+    uint16_t hi[8], lo[8];
 #pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const __half h = __float2half_rn(v[q]);
-      hi[i + q] = __half_as_ushort(h);
-      lo[i + q] = f16_bits(v[q] - __half2float(h));
+    for (int i = 0; i < 4; ++i) {
+      const int l = L - 1 - (kblock * (X2_KB / 2) + c16 * 4 + i);
+      float2 g = make_float2(0.f, 0.f);
+      if (l >= mp && b < n_items) g = __ldg(alm + (size_t)b * n_pairs + p0 + l - mp);
+      const float v[2] = {g.x * X2_PATTERN_SCALE, g.y * X2_PATTERN_SCALE};
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const __half h = __float2half_rn(v[q]);
+        hi[2 * i + q] = __half_as_ushort(h);
+        lo[2 * i + q] = f16_bits(v[q] - __half2float(h));
+      }
     }
+    uint8_t* p = blk + sw128(row, c16 * 8);
+    *(uint4*)p = pack8(hi);
+    *(uint4*)(p + X2_BLOCK) = pack8(lo);
   }
-  uint8_t* p = B + (size_t)(first + blk) * 2 * X2_BLOCK + sw128(row, c16 * 8);
-  *(uint4*)p = pack8(hi);
-  *(uint4*)(p + X2_BLOCK) = pack8(lo);
 }
 
 struct X2Args {
@@ -332,9 +333,8 @@ extern "C" int zeb_spectrum_x2(const float* alm, int n_items, const zeb_so3_dims
   a.kbmax = x2_kblocks(d->L, 0);
   a.stages = x2_stages(a.kbmax);
   a.inv = 1.f / (scale * X2_PATTERN_SCALE);
-  const long long chunks = (long long)a.ptiles * a.kbmax * 128 * 8;
-  const dim3 gp((unsigned)((chunks + 255) / 256), d->L);
-  k_x2_pack_patterns<<<gp, 256, 0, st>>>((const float2*)alm, n_items, d->n_pairs, d->L, a.ptiles, (uint8_t*)B);
+  const dim3 gp((unsigned)a.kbmax * a.ptiles, d->L);
+  k_x2_pack_patterns<<<gp, 256, 0, st>>>((const float2*)alm, n_items, d->n_pairs, d->L, a.ptiles, a.kbmax, (uint8_t*)B);
   int rc = zeb_launch_check("x2_pack_patterns");
   if (rc) return rc;
   ZEB_REQUIRE(((uintptr_t)U & 15) == 0, ZEB_EARG, "spectrum_x2: U must be 16-byte aligned");
