@@ -359,9 +359,6 @@ int zeb_records_fz_bunge(const float* records, int n, const double* ops, int n_o
 int zeb_det6(int mode, const float* pats, const float* items, int n, const zeb_frame_t* fr, const float* vpair,
              const float* gpair, int side, const float* x, const float* q0, float* out, void* stream);
 
-/* x[b] = A[b]⁻¹ b[b] for n systems of 6 (A: [n][6][6], b: [n][6], FP64) by elimination with
- * partial pivoting; ok[b] = 0 where a pivot falls below 1e-300 (x[b] = 0). Replaces the host
- * solve of planefit.zig:203-233 (the damped Levenberg–Marquardt step of settle). */
 /* zeb_det6 over the frame's masked-pixel list (zeb_mask_list, npix = zeb_mask_pixels entries, at
  * most 51200): 128 threads per pattern keep only the pattern's values in shared memory and
  * recompute each pixel's ray, so that four or five patterns share an SM; the same outputs. */
@@ -369,7 +366,21 @@ int zeb_det6_list(int mode, const float* pats, const float* items, int n, const 
                   int npix, const float* vpair, const float* gpair, int side, const float* x, const float* q0,
                   float* out, void* stream);
 
+/* x[b] = A[b]⁻¹ b[b] for n systems of 6 (A: [n][6][6], b: [n][6], FP64) by elimination with
+ * partial pivoting; ok[b] = 0 where a pivot falls below 1e-300 (x[b] = 0). Replaces the host
+ * solve of planefit.zig:203-233 (the damped Levenberg–Marquardt step of settle). */
 int zeb_solve6(const double* A, const double* b, int n, double* x, int* ok, void* stream);
+
+/* One round of the settle with six unknowns over n patterns (src/planefit.zig:570-622) from the sums of
+ * zeb_det6 mode 2 (width 43) or 3 (width 61: the adjoint's gradient) at (x, q0): each pattern's trial kept
+ * where its NCC rose and its λ adapted, then the next trial written to x [n][6] and q0 [n][4]. state:
+ * ZEB_SETTLE6_STATE doubles a pattern, [field][n]; before the first call (first != 0) its fields 29-32
+ * hold the starting orientation and x is zero, afterwards 0 is the NCC kept, 29-32 its orientation and
+ * 33-35 its shift. parts [(n + 31) / 32][3]: each 32 patterns' sum of NCC gained, the trials kept, and
+ * the trials lost with λ below 1e8. */
+#define ZEB_SETTLE6_STATE 44
+int zeb_settle6(const float* sums, int width, int n, double trust, int first, double* state, float* x, float* q0,
+                double* parts, void* stream);
 
 /* ── dictionary indexing ────────────────────────────────────────────────────────────────── */
 

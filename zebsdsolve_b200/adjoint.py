@@ -7,8 +7,8 @@ refine_orientation_projection_center).
 backward are the CUDA kernels of `zeb_det6` (mode 0 and mode 1); the backward recomputes the
 projection of every pixel from the parameters instead of keeping the projected patterns.
 `refine6` runs the reference's Levenberg–Marquardt settle over all the given patterns at once,
-with the damped 6 × 6 solve in FP64 on the device (`zeb_solve6`) and the Gauss–Newton matrix
-from the reference's 43 sums (`zeb_det6` mode 2); the gradient is the reference's (the gradient
+each round's verdicts and damped 6 × 6 solves in one FP64 kernel (`zeb_settle6`), the
+Gauss–Newton matrix from the reference's 43 sums (`zeb_det6` mode 2); the gradient is the reference's (the gradient
 table's) or the exact adjoint's (the kernel behind ProjectedNCC's backward).
 """
 import ctypes
@@ -74,25 +74,10 @@ def pc_jacobian(geo, rows, cols):
                     1)
 
 
-def _qmul(a, b):
-    aw, ax, ay, az = a.unbind(-1)
-    bw, bx, by, bz = b.unbind(-1)
-    return torch.stack([aw * bw - ax * bx - ay * by - az * bz, aw * bx + ax * bw + ay * bz - az * by,
-                        aw * by - ax * bz + ay * bw + az * bx, aw * bz + ax * by - ay * bx + az * bw], -1)
-
-
 def _qstd(q):
     n = torch.linalg.norm(q, dim=-1, keepdim=True)
     n = torch.where(n == 0, torch.ones_like(n), n)
     return q / n * torch.where(q[..., :1] < 0, -1.0, 1.0)
-
-
-def _exp(phi):
-    """rot.zig:192-198 — exp of rotation vectors."""
-    th2 = (phi * phi).sum(-1, keepdim=True)
-    th = torch.sqrt(th2)
-    k = torch.where(th < 1e-6, 0.5 - th2 / 48.0, torch.sin(0.5 * th) / torch.where(th < 1e-6, torch.ones_like(th), th))
-    return torch.cat([torch.cos(0.5 * th), k * phi], -1)
 
 
 def local_of(s):
@@ -143,50 +128,28 @@ def refine6(plan, q0, trust, most=60, gradient="reference"):
     Returns (q [n,4] f64, shift [n,3] f64 pixels, NCC [n], rounds)."""
     dev = q0.device
     n = plan.n
-    q = _qstd(q0.to(torch.float64))
-    shift = torch.zeros(n, 3, dtype=torch.float64, device=dev)
+    mode, width = (3, 61) if gradient == "adjoint" else (2, 43)
+    state = torch.zeros(N.ZEB_SETTLE6_STATE, n, dtype=torch.float64, device=dev)
+    state[29:33] = q0.t()
+    x = torch.zeros(n, 6, dtype=torch.float32, device=dev)
+    qf = _qstd(q0.to(torch.float64)).to(torch.float32).contiguous()
+    parts = torch.empty((n + 31) // 32, 3, dtype=torch.float64, device=dev)
 
-    def local(qq, ss):
-        x = torch.cat([ss, torch.zeros(n, 3, dtype=torch.float64, device=dev)], 1).to(torch.float32).contiguous()
-        qf = qq.to(torch.float32).contiguous()
-        if gradient == "adjoint":
-            # one pass: the GN sums and the adjoint's derivatives of the same projection
-            sums = plan.run(3, x, qf)
-            ok, ncc, _, H = local_of(sums[:, :43])
-            g = torch.where(ok[:, None], adjoint_gradient(sums), torch.zeros_like(H[:, 0]))
-            return ok, ncc, g, H
-        return local_of(plan.run(2, x, qf))
+    def step(first):
+        # the sums at (x, qf), then the round's verdicts and the next (x, qf)
+        N.call("zeb_settle6", ptr(plan.run(mode, x, qf)), width, n, float(trust), first, ptr(state), ptr(x), ptr(qf),
+               ptr(parts), stream_ptr())
 
-    keep = local(q, shift)
-    lam = torch.full((n,), 1e-3, dtype=torch.float64, device=dev)
+    step(1)
     count = max(n, 1)
-    eye = torch.eye(6, dtype=torch.float64, device=dev)
     rounds = 0
     while rounds < most:
-        H, g = keep[3], keep[2]
-        tr = torch.diagonal(H, dim1=1, dim2=2).sum(-1)
-        A = H + eye * (torch.diagonal(H, dim1=1, dim2=2) * lam[:, None])[:, :, None] + eye * (1e-9 * tr + 1e-30)[:, None, None]
-        A = A.contiguous()
-        b = g.contiguous()
-        d = torch.empty(n, 6, dtype=torch.float64, device=dev)
-        ok = torch.empty(n, dtype=torch.int32, device=dev)
-        N.call("zeb_solve6", ptr(A), ptr(b), n, ptr(d), ptr(ok), stream_ptr())
-        good = (ok != 0) & keep[0]
-        st = torch.where(good[:, None], torch.clamp(shift + d[:, :3], -trust, trust), shift)
-        qt = torch.where(good[:, None], _qstd(_qmul(_exp(d[:, 3:]), q)), q)
-        now = local(qt, st)
-        better = now[1] > keep[1]
-        gain = float(torch.where(better, now[1] - keep[1], torch.zeros_like(lam)).sum())
-        kept = int(better.sum())
-        damp = int((~better & (lam < 1e8)).sum())
-        q = torch.where(better[:, None], qt, q)
-        shift = torch.where(better[:, None], st, shift)
-        keep = tuple(torch.where(better.view(-1, *([1] * (k.dim() - 1))), nw, k) for k, nw in zip(keep, now))
-        lam = torch.where(better, torch.clamp(lam / 3, min=1e-4), torch.clamp(lam * 5, max=1e8))
+        step(0)
+        gain, kept, damp = parts.sum(0).tolist()
         if kept == 0 and damp > 0:  # (every step overshot: they go again, damped more)
             rounds += 1
             continue
         if gain / count < 1e-7:  # (the round that ends the loop is not counted, as the reference's)
             break
         rounds += 1
-    return q, shift, keep[1], rounds
+    return state[29:33].t().contiguous(), state[33:36].t().contiguous(), state[0], rounds

@@ -499,51 +499,205 @@ __global__ void __launch_bounds__(128, MODE == 3 ? 5 : 4) k_det6_list(Det6Args a
   det6_finish<MODE, NS>(a, b, s);
 }
 
-// x = A⁻¹ b for a (6 × 6, 6) system per item in FP64 (planefit.zig:203-233); ok[b] = 0 where a
-// pivot is below 1e-300 (x left 0).
-__global__ void k_solve6(const double* __restrict__ A, const double* __restrict__ bvec, int n, double* __restrict__ x,
-                         int* __restrict__ ok) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= n) return;
-  double M[36], r[6];
-  for (int i = 0; i < 36; ++i) M[i] = A[(size_t)b * 36 + i];
-  for (int i = 0; i < 6; ++i) r[i] = bvec[(size_t)b * 6 + i];
+// x = A⁻¹ b for a 6 × 6 system in FP64 by elimination with partial pivoting (planefit.zig:203-233), M and r
+// overwritten; false where a pivot is below 1e-300 (x then 0). Every index is a constant once unrolled,
+// so that the system stays in registers.
+__device__ __forceinline__ bool solve6(double (&M)[36], double (&r)[6], double (&x)[6]) {
   bool good = true;
-  for (int c = 0; c < 6 && good; ++c) {
+#pragma unroll
+  for (int c = 0; c < 6; ++c) {
     int piv = c;
+    double most = fabs(M[c * 6 + c]);
+#pragma unroll
     for (int rr = c + 1; rr < 6; ++rr)
-      if (fabs(M[rr * 6 + c]) > fabs(M[piv * 6 + c])) piv = rr;
-    if (fabs(M[piv * 6 + c]) < 1e-300) {
-      good = false;
-      break;
-    }
-    if (piv != c) {
-      for (int k = 0; k < 6; ++k) {
-        const double t = M[c * 6 + k];
-        M[c * 6 + k] = M[piv * 6 + k];
-        M[piv * 6 + k] = t;
+      if (fabs(M[rr * 6 + c]) > most) {
+        piv = rr;
+        most = fabs(M[rr * 6 + c]);
       }
-      const double t = r[c];
-      r[c] = r[piv];
-      r[piv] = t;
+    good = good && !(most < 1e-300);
+#pragma unroll
+    for (int rr = c + 1; rr < 6; ++rr) {
+      const bool swap = piv == rr;
+#pragma unroll
+      for (int k = c; k < 6; ++k) {
+        const double t = M[c * 6 + k], u = M[rr * 6 + k];
+        M[c * 6 + k] = swap ? u : t;
+        M[rr * 6 + k] = swap ? t : u;
+      }
+      const double t = r[c], u = r[rr];
+      r[c] = swap ? u : t;
+      r[rr] = swap ? t : u;
     }
+#pragma unroll
     for (int rr = c + 1; rr < 6; ++rr) {
       const double f = M[rr * 6 + c] / M[c * 6 + c];
       if (f == 0.0) continue;
+#pragma unroll
       for (int k = c; k < 6; ++k) M[rr * 6 + k] -= f * M[c * 6 + k];
       r[rr] -= f * r[c];
     }
   }
-  double y[6] = {0, 0, 0, 0, 0, 0};
-  if (good) {
-    for (int rr = 5; rr >= 0; --rr) {
-      double acc = r[rr];
-      for (int k = rr + 1; k < 6; ++k) acc -= M[rr * 6 + k] * y[k];
-      y[rr] = acc / M[rr * 6 + rr];
-    }
+#pragma unroll
+  for (int rr = 5; rr >= 0; --rr) {
+    double acc = r[rr];
+#pragma unroll
+    for (int k = rr + 1; k < 6; ++k) acc -= M[rr * 6 + k] * x[k];
+    x[rr] = acc / M[rr * 6 + rr];
   }
+  if (!good)
+#pragma unroll
+    for (int i = 0; i < 6; ++i) x[i] = 0.0;
+  return good;
+}
+
+__global__ void k_solve6(const double* __restrict__ A, const double* __restrict__ bvec, int n, double* __restrict__ x,
+                         int* __restrict__ ok) {
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b >= n) return;
+  double M[36], r[6], y[6];
+#pragma unroll
+  for (int i = 0; i < 36; ++i) M[i] = A[(size_t)b * 36 + i];
+#pragma unroll
+  for (int i = 0; i < 6; ++i) r[i] = bvec[(size_t)b * 6 + i];
+  const bool good = solve6(M, r, y);
+#pragma unroll
   for (int i = 0; i < 6; ++i) x[(size_t)b * 6 + i] = y[i];
   ok[b] = good ? 1 : 0;
+}
+
+// One round of the settle over every pattern (planefit.zig:570-622): the statistics of the sums just
+// evaluated (localOf, :176-200; the adjoint's gradient with 61 sums), the trial kept where its NCC rose
+// and λ adapted, then the next trial from what is kept: the damped 6 × 6 solve, the shift clamped to
+// ±trust, the rotation exp(d)·q. A thread a pattern, FP64 throughout; the state lies [S6_STATE][n] so
+// that neighbouring threads touch neighbouring words. A block's patterns' gain, kept and still-damped
+// counts go to parts[block][3], summed in a fixed order.
+// As ten dozen tensor operations a round this took 2.3 ms a round for 4096 patterns, nearly all of it
+// launches and three readbacks; here one launch and one readback. Blocks of 32 threads, since the
+// round is a serial chain in each thread and 4096 patterns are then 128 blocks on as many SMs.
+enum { S6_NCC = 0, S6_G = 1, S6_H = 7, S6_OK = 28, S6_Q = 29, S6_SHIFT = 33, S6_LAM = 36, S6_QT = 37, S6_ST = 41,
+       S6_STATE = 44 };
+
+__device__ __forceinline__ double clamp_d(double v, double lo, double hi) { return v < lo ? lo : (v > hi ? hi : v); }
+
+__device__ __forceinline__ void unit_up_d(double (&q)[4]) {  // unit, w >= 0 (0 stays 0)
+  double n = sqrt(q[0] * q[0] + q[1] * q[1] + q[2] * q[2] + q[3] * q[3]);
+  if (n == 0.0) n = 1.0;
+  const double sg = q[0] < 0.0 ? -1.0 : 1.0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) q[i] = q[i] / n * sg;
+}
+
+__global__ void __launch_bounds__(32) k_settle6(const float* __restrict__ sums, int width, int n, double trust, int first,
+                                                double* __restrict__ state, float* __restrict__ x,
+                                                float* __restrict__ q0, double* __restrict__ parts) {
+  const int b = blockIdx.x * 32 + threadIdx.x;
+  double gain = 0.0, kept = 0.0, damp = 0.0;
+  if (b < n) {
+    double* z = state + b;
+    const float* s = sums + (size_t)b * width;
+    const double cnt = fmax((double)s[0], 1.0);
+    const double mean = (double)s[1] / cnt;
+    const double var_n = (double)s[2] - cnt * mean * mean;
+    const bool ok = var_n > 1e-12;
+    const double inv = ok ? rsqrt(var_n) : 0.0;
+    const double ncc = ok ? (double)s[3] * inv : -2.0;
+    const double was = first ? 0.0 : z[(size_t)S6_NCC * n];
+    const bool better = first || ncc > was;
+    double q[4], sh[3], g[6], H[21], lam;
+    bool sound;
+    const int qo = first || !better ? S6_Q : S6_QT, so = first || !better ? S6_SHIFT : S6_ST;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) q[i] = z[(size_t)(qo + i) * n];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) sh[i] = first ? 0.0 : z[(size_t)(so + i) * n];
+    lam = first ? 1e-3 : z[(size_t)S6_LAM * n];
+    if (first) unit_up_d(q);
+    if (better) {
+      double au[6];
+      const int ds = width == 61 ? 43 : 4;  // the gradient's sums: the exact derivatives', or the table's
+#pragma unroll
+      for (int i = 0; i < 6; ++i) {
+        const double m = ((double)s[ds + 6 + i] - mean * (double)s[ds + i]) * inv;
+        g[i] = (ok || width != 61) ? ((double)s[ds + 12 + i] - ncc * m) * inv : 0.0;
+        au[i] = ((double)s[10 + i] - mean * (double)s[4 + i]) * inv;
+      }
+      int at = 0;
+#pragma unroll
+      for (int i = 0; i < 6; ++i)
+#pragma unroll
+        for (int j = i; j < 6; ++j, ++at)
+          H[at] = ((double)s[22 + at] - (double)s[4 + i] * (double)s[4 + j] / cnt - au[i] * au[j]) * (inv * inv);
+      sound = ok;
+      if (!first) {
+        gain = ncc - was;
+        kept = 1.0;
+        lam = fmax(lam / 3.0, 1e-4);
+      }
+      z[(size_t)S6_NCC * n] = ncc;
+      z[(size_t)S6_OK * n] = ok ? 1.0 : 0.0;
+#pragma unroll
+      for (int i = 0; i < 6; ++i) z[(size_t)(S6_G + i) * n] = g[i];
+#pragma unroll
+      for (int i = 0; i < 21; ++i) z[(size_t)(S6_H + i) * n] = H[i];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) z[(size_t)(S6_Q + i) * n] = q[i];
+#pragma unroll
+      for (int i = 0; i < 3; ++i) z[(size_t)(S6_SHIFT + i) * n] = sh[i];
+    } else {
+      sound = z[(size_t)S6_OK * n] != 0.0;
+#pragma unroll
+      for (int i = 0; i < 6; ++i) g[i] = z[(size_t)(S6_G + i) * n];
+#pragma unroll
+      for (int i = 0; i < 21; ++i) H[i] = z[(size_t)(S6_H + i) * n];
+      damp = lam < 1e8 ? 1.0 : 0.0;
+      lam = fmin(lam * 5.0, 1e8);
+    }
+    z[(size_t)S6_LAM * n] = lam;
+    // the next trial
+    double M[36], d[6];
+    double tr = 0.0;
+    int at = 0;
+#pragma unroll
+    for (int i = 0; i < 6; ++i)
+#pragma unroll
+      for (int j = i; j < 6; ++j, ++at) M[i * 6 + j] = M[j * 6 + i] = H[at];
+#pragma unroll
+    for (int i = 0; i < 6; ++i) tr += M[i * 7];
+#pragma unroll
+    for (int i = 0; i < 6; ++i) M[i * 7] = M[i * 7] + M[i * 7] * lam + (1e-9 * tr + 1e-30);
+    const bool good = solve6(M, g, d) && sound;
+    if (good) {
+#pragma unroll
+      for (int i = 0; i < 3; ++i) sh[i] = clamp_d(sh[i] + d[i], -trust, trust);
+      const double th2 = d[3] * d[3] + d[4] * d[4] + d[5] * d[5], th = sqrt(th2);
+      const double k = th < 1e-6 ? 0.5 - th2 / 48.0 : sin(0.5 * th) / th;
+      const double ew = cos(0.5 * th), ex = k * d[3], ey = k * d[4], ez = k * d[5];
+      double t[4] = {ew * q[0] - ex * q[1] - ey * q[2] - ez * q[3], ew * q[1] + ex * q[0] + ey * q[3] - ez * q[2],
+                     ew * q[2] - ex * q[3] + ey * q[0] + ez * q[1], ew * q[3] + ex * q[2] - ey * q[1] + ez * q[0]};
+      unit_up_d(t);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) q[i] = t[i];
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      z[(size_t)(S6_QT + i) * n] = q[i];
+      q0[(size_t)b * 4 + i] = (float)q[i];
+    }
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      z[(size_t)(S6_ST + i) * n] = sh[i];
+      x[(size_t)b * 6 + i] = (float)sh[i];
+      x[(size_t)b * 6 + 3 + i] = 0.f;
+    }
+  }
+  gain = warp_sum_d(gain);
+  kept = warp_sum_d(kept);
+  damp = warp_sum_d(damp);
+  if (threadIdx.x == 0) {
+    parts[blockIdx.x * 3 + 0] = gain;
+    parts[blockIdx.x * 3 + 1] = kept;
+    parts[blockIdx.x * 3 + 2] = damp;
+  }
 }
 
 }  // namespace zeb
@@ -659,4 +813,12 @@ extern "C" int zeb_solve6(const double* A, const double* b, int n, double* x, in
   if (n <= 0) return ZEB_OK;
   k_solve6<<<(n + 127) / 128, 128, 0, (cudaStream_t)stream>>>(A, b, n, x, ok);
   return zeb_launch_check("solve6");
+}
+
+extern "C" int zeb_settle6(const float* sums, int width, int n, double trust, int first, double* state, float* x,
+                           float* q0, double* parts, void* stream) {
+  ZEB_REQUIRE(sums && state && x && q0 && parts && (width == 43 || width == 61), ZEB_EARG, "settle6: bad arguments");
+  if (n <= 0) return ZEB_OK;
+  k_settle6<<<(n + 31) / 32, 32, 0, (cudaStream_t)stream>>>(sums, width, n, trust, first, state, x, q0, parts);
+  return zeb_launch_check("settle6");
 }
