@@ -651,13 +651,16 @@ class Engine:
             counts.append(total)
             grid = e
         cells = np.concatenate(lst)
+        # the list index of every cell, in a frame of none; the offsets are then one gather (its −1
+        # the 0xffffffff of no cell)
         r = R * P
+        wide = cols + 2 * r
+        framed = np.full((rows + 2 * r, wide), -1, np.int32)
+        framed[r:r + rows, r:r + cols] = index.reshape(rows, cols)
         off = np.arange(-r, r + 1)
-        y = (cells // cols)[:, None, None] + off[None, :, None]
-        x = (cells % cols)[:, None, None] + off[None, None, :]
-        inside = (y >= 0) & (y < rows) & (x >= 0) & (x < cols)
-        at = np.where(inside, index[np.clip(y, 0, rows - 1) * cols + np.clip(x, 0, cols - 1)], -1)
-        nbr = np.where(at >= 0, at, 0xFFFFFFFF).astype(np.uint32).reshape(len(cells), -1)
+        slots = (off[:, None] * wide + off[None, :]).reshape(-1)
+        at = (cells // cols + r) * wide + cells % cols + r
+        nbr = framed.reshape(-1)[at[:, None] + slots[None, :]].view(np.uint32)
         return cells, counts, nbr
 
     def nlpar_average(self, cells, account=False):
@@ -716,19 +719,15 @@ class Engine:
         patterns' noise (a pixel's standard deviation), the share of it an average keeps and the
         share of an average that is the pattern itself, each a mean over the cells."""
         s = self.set
-        noise = kept = own = counted = 0.0
-        for c in range(n):
-            sh_ = shares[c * F:(c + 1) * F].astype(np.float64)
-            nb = nbr[c]
-            inside = nb != 0xFFFFFFFF
-            before = float(sig[c])
-            after = float((sh_[inside] ** 2 * sig[nb[inside].astype(np.int64)]).sum())
-            own += sh_[F // 2]
-            if not before > 0:
-                continue
-            noise += math.sqrt(before)
-            kept += math.sqrt(after / before)
-            counted += 1
+        sh_ = shares[:n * F].reshape(n, F).astype(np.float64)
+        inside = nbr[:n] != 0xFFFFFFFF
+        before = sig[:n].astype(np.float64)
+        after = np.where(inside, sh_ ** 2 * sig[np.where(inside, nbr[:n], 0)], 0.0).sum(1)
+        own = float(sh_[:, F // 2].sum())
+        some = before > 0
+        counted = int(some.sum())
+        noise = float(np.sqrt(before[some]).sum())
+        kept = float(np.sqrt(after[some] / before[some]).sum())
         P, R = int(s["nlpar_iterations"]), int(s["nlpar_radius"])
         self.log(f"neighbour averaging: {P} pass{'' if P == 1 else 'es'} over {2 * R + 1} × {2 * R + 1} cells "
                  f"(λ {s['nlpar_lambda']:.2f}); noise about {noise / max(counted, 1):.2f} a pixel, "
