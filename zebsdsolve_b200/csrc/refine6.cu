@@ -250,7 +250,7 @@ __device__ __forceinline__ float4 grad_and_slope(const float* __restrict__ gp, f
 // R⁻¹·∇M/|v|, are summed in the turned frame as ∇M/|v| (det6_unturn takes the sums back once a
 // pattern: R⁻¹ on the vectors, R⁻¹·(·)·R and R⁻¹·(·) on the blocks of products); those along the
 // rotation, c × ∇M, need no turning.
-template <int MODE, int NS>
+template <int MODE, int NS, bool SMOOTH = false>
 __device__ __forceinline__ void det6_pixel(const Det6Args& a, float3 rv, float e, float (&s)[NS]) {
   const float inv = rsqrtf(dot3(rv, rv));  // 1/|v|
   const float3 c = make_float3(rv.x * inv, rv.y * inv, rv.z * inv);
@@ -263,9 +263,9 @@ __device__ __forceinline__ void det6_pixel(const Det6Args& a, float3 rv, float e
     if (MODE == 1) {
       m = master_and_slope(a.vpair, c, a.side, g);
     } else if (MODE == 2) {
-      const float4 gm = a.interp == 0   ? grad_at_pair(a.gpair, c, a.side)
-                        : a.interp == 1 ? grad_smooth<1>(a.sheets, c, a.side)
-                                        : grad_smooth<2>(a.sheets, c, a.side);
+      float4 gm;
+      if (!SMOOTH) gm = grad_at_pair(a.gpair, c, a.side);
+      else gm = a.interp == 1 ? grad_smooth<1>(a.sheets, c, a.side) : grad_smooth<2>(a.sheets, c, a.side);
       m = gm.w;
       g = make_float3(gm.x, gm.y, gm.z);
     } else {
@@ -439,29 +439,27 @@ __global__ void __launch_bounds__(256) k_det6(Det6Args a) {
   det6_finish<MODE, NS>(a, b, s);
 }
 
-// The same over the frame's masked-pixel list (zeb_mask_list, shared by every pattern): 128
-// threads per pattern keep only the pattern's values along the list in shared memory and
-// recompute each pixel's ray, so that several patterns share an SM (a list of (ray, value) per
-// block fills an SM's shared memory for one 120 × 120 pattern).
-// (the one-pass mode: five blocks an SM at 96 registers, one pixel a thread at a time, measured
-// 11 % faster than four blocks with two pixels in flight: the table loads' latency is hidden by
-// the warps rather than by unrolling; the other modes keep four blocks, which mode 2's smooth
-// kernels need to run without spilling)
-template <int MODE>
-__global__ void __launch_bounds__(128, MODE == 3 ? 5 : 4) k_det6_list(Det6Args a, const uint32_t* __restrict__ list,
-                                                                     int npix) {
+// The same over the frame's masked-pixel list (zeb_mask_list, shared by every pattern): 128 threads per
+// pattern recompute each pixel's ray. What bounds it is the latency of the table's loads (32 or 64
+// gathered bytes a pixel), so the pattern's values, read once and in order, come straight from memory
+// and shared memory stays empty: staging them first cost a pass before the sums, limited an SM to four
+// patterns of 120 × 120 and left the loads no cache, where a detector's neighbouring rows share the
+// table's rows. 4096 patterns of 120 × 120, modes 0-3: 737, 732, 842, 970 → 244, 416, 611, 689 µs; 1024
+// of 160 × 160: 569, 650, 657, 781 → 142, 226, 298, 342. One pixel a thread at a time where the sums
+// are many: their registers then leave no room for two (mode 3 with two in flight 799 µs at four
+// blocks an SM; mode 2 at five blocks 579 µs at 120 × 120, but 331 at 160 × 160).
+// SMOOTH: mode 2 with the smooth kernels, by themselves so that the bilinear mode does not carry
+// their registers.
+template <int MODE, bool SMOOTH = false>
+__global__ void __launch_bounds__(128, MODE <= 1 ? 8 : 4) k_det6_list(Det6Args a, const uint32_t* __restrict__ list,
+                                                                         int npix) {
   constexpr int NS = MODE == 0 ? 4 : (MODE == 1 ? 22 : (MODE == 2 ? 43 : 61));
-  extern __shared__ float pv6[];
   __shared__ float red[NS * 4];
   __shared__ float4 sh_q;
   __shared__ float3 sh_t;
   const int b = blockIdx.x;
   const float4 it = a.items[b];
   const float* gpat = a.pats + (size_t)(int)it.w * a.h * a.w;
-  for (int k = threadIdx.x; k < npix; k += blockDim.x) {
-    const uint32_t v = __ldg(list + k);
-    pv6[k] = __ldg(gpat + (int)(v >> 16) * a.w + (int)(v & 0xffffu));
-  }
   if (threadIdx.x == 0) {
     const float* x = a.x + (size_t)b * 6;
     const float* q0 = a.q0 + (size_t)b * 4;
@@ -481,12 +479,13 @@ __global__ void __launch_bounds__(128, MODE == 3 ? 5 : 4) k_det6_list(Det6Args a
   for (int k = 0; k < NS; ++k) s[k] = 0.f;
   auto pixel = [&](int k) {
     const uint32_t v = __ldg(list + k);
+    const float e = __ldg(gpat + (int)(v >> 16) * a.w + (int)(v & 0xffffu));
     const float row = (float)(int)(v >> 16), col = (float)(int)(v & 0xffffu);
     const float3 rv = make_float3(fmaf(rc0.x, row, fmaf(rc1.x, col, rt.x)), fmaf(rc0.y, row, fmaf(rc1.y, col, rt.y)),
                                   fmaf(rc0.z, row, fmaf(rc1.z, col, rt.z)));
-    det6_pixel<MODE, NS>(a, rv, pv6[k], s);
+    det6_pixel<MODE, NS, SMOOTH>(a, rv, e, s);
   };
-  if constexpr (MODE == 3) {
+  if constexpr (MODE >= 2) {
 #pragma unroll 1
     for (int k = threadIdx.x; k < npix; k += blockDim.x) pixel(k);
   } else {
@@ -751,8 +750,7 @@ extern "C" int zeb_det6_list(int mode, const float* pats, const float* items, in
               "det6_list: pair tables misaligned");
   ZEB_REQUIRE(npix == zeb_mask_count(fr), ZEB_EARG, "det6_list: %d pixels listed, the frame masks %d", npix,
               zeb_mask_count(fr));
-  const size_t smem = (size_t)npix * sizeof(float);
-  ZEB_REQUIRE(npix >= 1 && smem <= 200 * 1024, ZEB_ESIZE, "det6_list: %d pixels (at most 51200)", npix);
+  ZEB_REQUIRE(npix >= 1 && npix <= 51200, ZEB_ESIZE, "det6_list: %d pixels (at most 51200)", npix);
   if (n <= 0) return ZEB_OK;
   Det6Args a{};
   ZEB_REQUIRE(fr->h >= 2 && fr->w >= 2 && fr->h < 65536 && fr->w < 65536, ZEB_EARG, "det6_list: bad frame");
@@ -765,17 +763,13 @@ extern "C" int zeb_det6_list(int mode, const float* pats, const float* items, in
   a.side = side; a.x = x; a.q0 = q0; a.out = out;
   cudaStream_t st = (cudaStream_t)stream;
   if (mode == 0) {
-    if (smem > 48 * 1024) cudaFuncSetAttribute(k_det6_list<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_det6_list<0><<<n, 128, smem, st>>>(a, list, npix);
+    k_det6_list<0><<<n, 128, 0, st>>>(a, list, npix);
   } else if (mode == 1) {
-    if (smem > 48 * 1024) cudaFuncSetAttribute(k_det6_list<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_det6_list<1><<<n, 128, smem, st>>>(a, list, npix);
+    k_det6_list<1><<<n, 128, 0, st>>>(a, list, npix);
   } else if (mode == 2) {
-    if (smem > 48 * 1024) cudaFuncSetAttribute(k_det6_list<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_det6_list<2><<<n, 128, smem, st>>>(a, list, npix);
+    k_det6_list<2><<<n, 128, 0, st>>>(a, list, npix);
   } else {
-    if (smem > 48 * 1024) cudaFuncSetAttribute(k_det6_list<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_det6_list<3><<<n, 128, smem, st>>>(a, list, npix);
+    k_det6_list<3><<<n, 128, 0, st>>>(a, list, npix);
   }
   return zeb_launch_check("det6_list");
 }
@@ -790,8 +784,7 @@ extern "C" int zeb_sums6_list(const float* pats, const float* items, int n, cons
   ZEB_REQUIRE(((uintptr_t)gpair & 31) == 0, ZEB_EARG, "sums6_list: gradient pairs misaligned");
   ZEB_REQUIRE(npix == zeb_mask_count(fr), ZEB_EARG, "sums6_list: %d pixels listed, the frame masks %d", npix,
               zeb_mask_count(fr));
-  const size_t smem = (size_t)npix * sizeof(float);
-  ZEB_REQUIRE(npix >= 1 && smem <= 200 * 1024, ZEB_ESIZE, "sums6_list: %d pixels (at most 51200)", npix);
+  ZEB_REQUIRE(npix >= 1 && npix <= 51200, ZEB_ESIZE, "sums6_list: %d pixels (at most 51200)", npix);
   if (n <= 0) return ZEB_OK;
   Det6Args a{};
   ZEB_REQUIRE(fr->h >= 2 && fr->w >= 2 && fr->h < 65536 && fr->w < 65536, ZEB_EARG, "sums6_list: bad frame");
@@ -803,8 +796,8 @@ extern "C" int zeb_sums6_list(const float* pats, const float* items, int n, cons
   a.pats = pats; a.items = (const float4*)items; a.n = n; a.gpair = gpair; a.sheets = sheets; a.interp = interp;
   a.side = side; a.x = x; a.q0 = q0; a.out = out;
   cudaStream_t st = (cudaStream_t)stream;
-  if (smem > 48 * 1024) cudaFuncSetAttribute(k_det6_list<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  k_det6_list<2><<<n, 128, smem, st>>>(a, list, npix);
+  if (interp == 0) k_det6_list<2><<<n, 128, 0, st>>>(a, list, npix);
+  else k_det6_list<2, true><<<n, 128, 0, st>>>(a, list, npix);
   return zeb_launch_check("sums6_list");
 }
 
