@@ -566,30 +566,42 @@ static size_t det_smem(DetArgs& a) {
 // ── the refinement over a precomputed pixel list ──
 //
 // The frame's masked pixels, in raster order, come as one list shared by every item (packed
-// (row << 16) | col, zeb_mask_list); a block of 128 threads per item keeps only the pattern's
-// values along the list in shared memory (4 bytes a pixel, 8 with NMI's simulated values), so
-// that six items share an SM and one item's serial phase (the reduction and thread 0's step)
-// overlaps the others' pixel passes (256 or 512 threads where those values pass 36 or 72 KB, so
-// that the warps an SM holds stay about as many for a large detector's list).  Each pass recomputes the detector ray of every pixel (nine
-// FMAs and a reciprocal square root) instead of keeping it; the sums per pixel are those of
-// k_refine.
+// (row << 16) | col, zeb_mask_list); a block of 128 threads per item, so that seven items share an SM
+// and one item's serial phase (the reduction and thread 0's step) overlaps the others' pixel passes
+// (256 or 512 threads for the long list of a large detector, so that the warps an SM holds stay about
+// as many). Each pass recomputes the detector ray of every pixel (nine FMAs and a reciprocal square
+// root) instead of keeping it, and reads the pattern's values in order from memory; shared memory holds
+// the NMI's simulated values alone. The sums per pixel are those of k_refine.
+//
+// What bounds it: the latency of the table's gathered loads (32 bytes a pixel in FP16, 64 in FP32, from
+// L2: one warp instruction in two cycles issues at 18 warps an SM), so what counts is the warps an SM
+// holds. With the pattern's values in shared memory too (8 bytes a pixel) and the refinement's state in
+// every thread's registers, six items an SM, three at 256 threads and one at 512: eleven passes over
+// 16384 patterns of 60 × 60 4.95 → 4.51 ms in FP32, 3.71 → 3.37 in FP16; 2048 of 96 × 96 1.61 → 1.48 and
+// 1.19 → 1.14; 1024 of 120 × 160 1.37 → 1.20 and 1.22 → 0.94. (Eight items of 128 threads with two pixels
+// in flight a thread instead of four: 4.48 and 3.39, but 300 patterns 0.191 → 0.234.)
 
-// the block size for a list whose pattern values and simulated values take `smem` bytes
-inline int rl_threads(size_t smem) { return smem <= 36 * 1024 ? 128 : (smem <= 72 * 1024 ? 256 : 512); }
+// the block size for a list of npix pixels: a longer one leaves fewer items an SM
+inline int rl_threads(int npix) { return npix <= 4608 ? 128 : (npix <= 9216 ? 256 : 512); }
 
 __device__ __forceinline__ float3 list_ray(const DetArgs& a, float3 t, uint32_t v) {
   return ray_dir(a, t, (int)(v >> 16), (int)(v & 0xffffu));
 }
 
-// the NMI over the list (detector.wgsl:744-832); sims (shared, npix floats) keeps the simulated
-// values of the first pass for the histogram pass
-__device__ float nmi_list(const DetArgs& a, const uint32_t* __restrict__ list, const float* pv, float* sims,
+__device__ __forceinline__ float list_value(const DetArgs& a, const float* __restrict__ gpat, uint32_t v) {
+  return __ldg(gpat + (int)(v >> 16) * a.w + (int)(v & 0xffffu));
+}
+
+// the NMI over the list (detector.wgsl:744-832) of the pattern gpat; sims (shared, npix floats) keeps the
+// simulated values of the first pass for the histogram pass
+__device__ float nmi_list(const DetArgs& a, const uint32_t* __restrict__ list, const float* __restrict__ gpat, float* sims,
                           int npix, float3 t, float4 q, int nbins, uint32_t* hist, float* red) {
   float ext[4] = {3.4e38f, -3.4e38f, 3.4e38f, -3.4e38f};
 #pragma unroll 4
   for (int k = threadIdx.x; k < npix; k += blockDim.x) {
-    const float e = pv[k];
-    const float sv = master_at_pair(a.vpair, qrot(q, list_ray(a, t, __ldg(list + k))), a.side);
+    const uint32_t v = __ldg(list + k);
+    const float e = list_value(a, gpat, v);
+    const float sv = master_at_pair(a.vpair, qrot(q, list_ray(a, t, v)), a.side);
     sims[k] = sv;
     ext[0] = fminf(ext[0], e); ext[1] = fmaxf(ext[1], e);
     ext[2] = fminf(ext[2], sv); ext[3] = fmaxf(ext[3], sv);
@@ -615,7 +627,8 @@ __device__ float nmi_list(const DetArgs& a, const uint32_t* __restrict__ list, c
   const float ke = (float)nbins / fmaxf(r[1] - r[0], 1e-20f);
   const float ks = (float)nbins / fmaxf(r[3] - r[2], 1e-20f);
   for (int k = threadIdx.x; k < npix; k += blockDim.x) {
-    const uint32_t be = min((uint32_t)((pv[k] - r[0]) * ke), (uint32_t)(nbins - 1));
+    const uint32_t v = __ldg(list + k);
+    const uint32_t be = min((uint32_t)((list_value(a, gpat, v) - r[0]) * ke), (uint32_t)(nbins - 1));
     const uint32_t bs = min((uint32_t)((sims[k] - r[2]) * ks), (uint32_t)(nbins - 1));
     atomicAdd(&hist[be * nbins + bs], 1u);
   }
@@ -642,32 +655,37 @@ __device__ float nmi_list(const DetArgs& a, const uint32_t* __restrict__ list, c
   return h_marg > 1e-12f ? 2.f * (h_marg - h_joint) / h_marg : 0.f;
 }
 
+struct RefineState {
+  float4 q_best;
+  float best, mu, g_best[3], h_best[6], last_good, promised, step_len, accepted;
+};
+
 // QUAD: the lookups from the FP16 neighbourhood records (a.gpair holds zeb_master_quads' table)
-// TH threads a pattern: 128 (six patterns an SM) while the list is small; a list whose shared
-// memory leaves fewer blocks an SM takes 256 or 512, so that an SM keeps its warps
+// TH threads a pattern: 128 (seven patterns an SM) while the list is small; a long list takes 256 or
+// 512, so that its serial phases stay short beside its passes
 template <bool QUAD, int TH>
-__global__ void __launch_bounds__(TH, TH == 128 ? 6 : (TH == 256 ? 3 : 1)) k_refine_list(DetArgs a, const uint32_t* __restrict__ list,
-                                                                 int npix) {
-  extern __shared__ float pv[];  // [npix] pattern values, then [npix] simulated values (NMI)
+__global__ void __launch_bounds__(TH, TH == 128 ? 7 : (TH == 256 ? 4 : 2))
+    k_refine_list(DetArgs a, const uint32_t* __restrict__ list, int npix) {
+  extern __shared__ float sims[];  // [npix] simulated values (NMI)
   __shared__ float red[20 * (TH / 32)];
   __shared__ uint32_t hist[32 * 32];
   __shared__ float4 sh_q;
+  __shared__ RefineState st;
   const int b = blockIdx.x;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   constexpr int NW = TH / 32;
   const float4 it = a.items[b];
   const float3 t = make_float3(it.x, it.y, it.z);
   const float* gpat = a.pats + (size_t)(int)it.w * a.h * a.w;
-  for (int k = threadIdx.x; k < npix; k += TH) {
-    const uint32_t v = __ldg(list + k);
-    pv[k] = __ldg(gpat + (int)(v >> 16) * a.w + (int)(v & 0xffffu));
+  // refinement state (thread 0's, in shared memory): detector.wgsl:73-77
+  if (threadIdx.x == 0) {
+    const float* sd0 = a.seeds + (size_t)b * a.seed_stride;
+    st = RefineState{};
+    st.q_best = make_float4(sd0[0], sd0[1], sd0[2], sd0[3]);
+    st.best = -2.f;
+    st.mu = a.o.scale0;
+    sh_q = st.q_best;
   }
-  // refinement state (thread 0's registers): detector.wgsl:73-77
-  const float* sd0 = a.seeds + (size_t)b * a.seed_stride;
-  float4 q_best = make_float4(sd0[0], sd0[1], sd0[2], sd0[3]);
-  float best = -2.f, mu = a.o.scale0, g_best[3] = {0.f, 0.f, 0.f}, h_best[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  float last_good = 0.f, promised = 0.f, step_len = 0.f, accepted = 0.f;
-  if (threadIdx.x == 0) sh_q = q_best;
   __syncthreads();
 
   for (int iter = 0; iter <= a.o.iters; ++iter) {
@@ -677,7 +695,7 @@ __global__ void __launch_bounds__(TH, TH == 128 ? 6 : (TH == 256 ? 3 : 1)) k_ref
     float s[19];
 #pragma unroll
     for (int k = 0; k < 19; ++k) s[k] = 0.f;
-#pragma unroll 4
+#pragma unroll (TH == 128 ? 4 : 2)
     for (int k = threadIdx.x; k < npix; k += TH) {
       const uint32_t v = __ldg(list + k);
       const float row = (float)(int)(v >> 16), col = (float)(int)(v & 0xffffu);
@@ -686,7 +704,7 @@ __global__ void __launch_bounds__(TH, TH == 128 ? 6 : (TH == 256 ? 3 : 1)) k_ref
                                               fmaf(rc0.z, row, fmaf(rc1.z, col, rt.z))));
       const float4 m = QUAD ? grad_at_quad(a.gpair, c, a.side) : grad_at_pair(a.gpair, c, a.side);
       const float3 d = cross3(c, make_float3(m.x, m.y, m.z));
-      const float e = pv[k];
+      const float e = list_value(a, gpat, v);
       s[1] += m.w; s[2] += m.w * m.w; s[3] += m.w * e;
       s[4] += d.x; s[5] += d.y; s[6] += d.z;
       s[7] += m.w * d.x; s[8] += m.w * d.y; s[9] += m.w * d.z;
@@ -733,19 +751,22 @@ __global__ void __launch_bounds__(TH, TH == 128 ? 6 : (TH == 256 ? 3 : 1)) k_ref
       for (int k = 1; k < 19; ++k) s[k] = __shfl_sync(0xffffffffu, tot, k);
       s[0] = (float)npix;
       if (lane == 0) {
-        float4 qn = q_best;
-        refine_step(a.o, iter, q, s, best, mu, g_best, h_best, last_good, promised, step_len, accepted, q_best, qn);
+        RefineState z = st;
+        float4 qn = z.q_best;
+        refine_step(a.o, iter, q, s, z.best, z.mu, z.g_best, z.h_best, z.last_good, z.promised, z.step_len, z.accepted,
+                    z.q_best, qn);
+        st = z;
         sh_q = qn;
       }
     }
     __syncthreads();
   }
   const float4 qf = sh_q;
-  const float v = nmi_list(a, list, pv, pv + npix, npix, t, qf, a.o.nmi_bins, hist, red);
+  const float v = nmi_list(a, list, gpat, sims, npix, t, qf, a.o.nmi_bins, hist, red);
   if (threadIdx.x == 0) {
     float* r = a.records + (size_t)b * 8;
     r[0] = qf.x; r[1] = qf.y; r[2] = qf.z; r[3] = qf.w;
-    r[4] = best; r[5] = v; r[6] = last_good; r[7] = a.o.stamp;
+    r[4] = st.best; r[5] = v; r[6] = st.last_good; r[7] = a.o.stamp;
   }
 }
 
@@ -775,17 +796,19 @@ __global__ void k_mask_list(DetArgs a, uint32_t* __restrict__ list) {
 }
 
 template <bool QUAD, int TH>
-void rl_launch_th(const DetArgs& a, const uint32_t* list, int npix, size_t smem, cudaStream_t st) {
-  if (smem > 48 * 1024) cudaFuncSetAttribute(k_refine_list<QUAD, TH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+void rl_launch_th(const DetArgs& a, const uint32_t* list, int npix, cudaStream_t st) {
+  const size_t smem = (size_t)npix * sizeof(float);
+  if (smem > 40 * 1024)  // (beside the static 5 KB)
+    cudaFuncSetAttribute(k_refine_list<QUAD, TH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   k_refine_list<QUAD, TH><<<a.n, TH, smem, st>>>(a, list, npix);
 }
 
 template <bool QUAD>
-void rl_launch(const DetArgs& a, const uint32_t* list, int npix, size_t smem, cudaStream_t st) {
-  const int th = rl_threads(smem);
-  if (th == 128) rl_launch_th<QUAD, 128>(a, list, npix, smem, st);
-  else if (th == 256) rl_launch_th<QUAD, 256>(a, list, npix, smem, st);
-  else rl_launch_th<QUAD, 512>(a, list, npix, smem, st);
+void rl_launch(const DetArgs& a, const uint32_t* list, int npix, cudaStream_t st) {
+  const int th = rl_threads(npix);
+  if (th == 128) rl_launch_th<QUAD, 128>(a, list, npix, st);
+  else if (th == 256) rl_launch_th<QUAD, 256>(a, list, npix, st);
+  else rl_launch_th<QUAD, 512>(a, list, npix, st);
 }
 
 }  // namespace zeb
@@ -852,7 +875,7 @@ extern "C" int zeb_refine_list(const float* pats, const float* items, const floa
   ZEB_REQUIRE(fill_frame(a, fr), ZEB_EARG, "refine_list: bad frame");
   a.pats = pats; a.items = (const float4*)items; a.seeds = seeds; a.seed_stride = seed_stride; a.n = n;
   a.vpair = (const float2*)vpair; a.gpair = gpair; a.side = side; a.o = *o; a.records = records;
-  rl_launch<false>(a, list, npix, smem, (cudaStream_t)stream);
+  rl_launch<false>(a, list, npix, (cudaStream_t)stream);
   return zeb_launch_check("refine_list");
 }
 
@@ -877,7 +900,7 @@ extern "C" int zeb_refine_list_h(const float* pats, const float* items, const fl
   ZEB_REQUIRE(fill_frame(a, fr), ZEB_EARG, "refine_list_h: bad frame");
   a.pats = pats; a.items = (const float4*)items; a.seeds = seeds; a.seed_stride = seed_stride; a.n = n;
   a.vpair = (const float2*)vpair; a.gpair = (const float*)quads; a.side = side; a.o = *o; a.records = records;
-  rl_launch<true>(a, list, npix, smem, (cudaStream_t)stream);
+  rl_launch<true>(a, list, npix, (cudaStream_t)stream);
   return zeb_launch_check("refine_list_h");
 }
 
