@@ -1,0 +1,45 @@
+"""The correlation's transform along a with the next slab on its way (k_slab_stream: 32 columns of 64 points
+to a slab, one denominator volume) against the kernel that holds its loads in registers (k_slab_cols, which
+U on an 8-byte boundary takes): the same arithmetic in the same order, so the same bits (GPU only).
+"""
+import ctypes
+
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+def _p(t):
+    return ctypes.c_void_p(t.data_ptr())
+
+
+@pytest.mark.parametrize("L,n", [(64, 1), (64, 13), (33, 200), (63, 77), (48, 300), (64, 700)])
+def test_streamed_slabs_give_the_same_peaks(L, n):
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from zebsdsolve_b200 import _native as N
+
+    d = N.So3Dims(L, 128, 65, 32, 4, (L - 1) // 4, L * (L + 1) // 2)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(L * 1000 + n)
+    count = n * 65 * L * 32 * 2
+    both = torch.empty(count + 4, device="cuda")
+    U = torch.randn(count, device="cuda", generator=g)
+    rden = torch.rand(65 * 32 * 128, device="cuda", generator=g) + 0.5
+    rden[::13] = 0
+    t = -2j * torch.pi * torch.arange(1024, dtype=torch.float64) / 1024
+    tw = torch.view_as_real(torch.exp(t).to(torch.complex64)).contiguous().cuda()
+    got = []
+    for shift in (0, 2):  # floats: a 16-byte boundary, and an 8-byte one
+        u = both[shift:shift + count]
+        u.copy_(U)
+        assert u.data_ptr() % 16 == 4 * shift
+        scratch = torch.empty(N.load().zeb_peaks_scratch_bytes(ctypes.byref(d), n), dtype=torch.uint8, device="cuda")
+        peaks = torch.zeros(n, 8, device="cuda")
+        N.call("zeb_correlate_peaks", _p(u), n, ctypes.byref(d), _p(tw), _p(rden), 1 << 30, _p(peaks), _p(scratch),
+               ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+        torch.cuda.synchronize()
+        got.append((peaks, scratch[: n * 65 * 8].clone()))
+    assert torch.equal(got[0][1], got[1][1])
+    assert torch.equal(got[0][0], got[1][0])

@@ -175,6 +175,46 @@ __device__ __forceinline__ void fft_reg(float2 (&x)[N]) {
   }
 }
 
+// a column's values from its coefficients z (0 beyond L) and row rd of rden: the largest kept in
+// (bv, bi), the first of equal ones (base: the column's first volume index)
+template <int H>
+__device__ __forceinline__ void column_best(float2 (&z)[H], const float4* rd, uint32_t base, float& bv, uint32_t& bi) {
+  // Z_q = (X_q + X_{q+h}) + i w_q (X_q − X_{q+h}), X_{q+h} = conj X_{h−q}, w_q = e^{−2πi q/n},
+  // computed for q and h − q together from the same two points (in place)
+#pragma unroll
+  for (int q = 0; q <= H / 2; ++q) {
+    const int qm = (H - q) & (H - 1);
+    float2 xq = z[q], xm = z[qm];
+    float2 zq;
+    {
+      float2 x = xq, y = make_float2(0.f, 0.f);
+      if (q == 0) x.y = 0.f;
+      else y = make_float2(xm.x, -xm.y);
+      const float2 w = tw_of<2 * H>(q);
+      const float2 dd = make_float2(x.x - y.x, x.y - y.y);
+      zq = make_float2(x.x + y.x - (w.x * dd.y + w.y * dd.x), x.y + y.y + (w.x * dd.x - w.y * dd.y));
+    }
+    if (q != 0 && qm != q) {
+      float2 x = xm, y = make_float2(xq.x, -xq.y);
+      const float2 w = tw_of<2 * H>(qm);
+      const float2 dd = make_float2(x.x - y.x, x.y - y.y);
+      z[qm] = make_float2(x.x + y.x - (w.x * dd.y + w.y * dd.x), x.y + y.y + (w.x * dd.x - w.y * dd.y));
+    }
+    z[q] = zq;
+  }
+  fft_reg<H>(z);
+#pragma unroll
+  for (int p = 0; p < H; p += 2) {
+    const float4 r = rd[p / 2];
+    const float v0 = z[p].x * r.x, v1 = z[p].y * r.y, v2 = z[p + 1].x * r.z, v3 = z[p + 1].y * r.w;
+    const uint32_t i0 = base + 2 * p;
+    if (v0 > bv) { bv = v0; bi = i0; }
+    if (v1 > bv) { bv = v1; bi = i0 + 1; }
+    if (v2 > bv) { bv = v2; bi = i0 + 2; }
+    if (v3 > bv) { bv = v3; bi = i0 + 3; }
+  }
+}
+
 // rden rows of one j staged per warp (rows padded by 4 floats: the lanes' 16-byte reads of
 // their own rows fall in distinct banks)
 template <int NC, int H>
@@ -263,42 +303,7 @@ __global__ void __launch_bounds__(WARPS * 32, PER_SM) k_slab_cols(SlabArgs a) {
       float2 z[H];
 #pragma unroll
       for (int q = 0; q < H; ++q) z[q] = q < L ? __ldcs(src + q * NC + c) : make_float2(0.f, 0.f);
-      // Z_q = (X_q + X_{q+h}) + i w_q (X_q − X_{q+h}), X_{q+h} = conj X_{h−q}, w_q = e^{−2πi q/n},
-      // computed for q and h − q together from the same two points (in place)
-#pragma unroll
-      for (int q = 0; q <= H / 2; ++q) {
-        const int qm = (H - q) & (H - 1);
-        float2 xq = z[q], xm = z[qm];
-        float2 zq;
-        {
-          float2 x = xq, y = make_float2(0.f, 0.f);
-          if (q == 0) x.y = 0.f;
-          else y = make_float2(xm.x, -xm.y);
-          const float2 w = tw_of<2 * H>(q);
-          const float2 dd = make_float2(x.x - y.x, x.y - y.y);
-          zq = make_float2(x.x + y.x - (w.x * dd.y + w.y * dd.x), x.y + y.y + (w.x * dd.x - w.y * dd.y));
-        }
-        if (q != 0 && qm != q) {
-          float2 x = xm, y = make_float2(xq.x, -xq.y);
-          const float2 w = tw_of<2 * H>(qm);
-          const float2 dd = make_float2(x.x - y.x, x.y - y.y);
-          z[qm] = make_float2(x.x + y.x - (w.x * dd.y + w.y * dd.x), x.y + y.y + (w.x * dd.x - w.y * dd.y));
-        }
-        z[q] = zq;
-      }
-      fft_reg<H>(z);
-      const float4* rd = (const float4*)(rslab + (size_t)c * rstride);
-      const uint32_t base = ((uint32_t)(j * NC + c)) * n;
-#pragma unroll
-      for (int p = 0; p < H; p += 2) {
-        const float4 r = rd[p / 2];
-        const float v0 = z[p].x * r.x, v1 = z[p].y * r.y, v2 = z[p + 1].x * r.z, v3 = z[p + 1].y * r.w;
-        const uint32_t i0 = base + 2 * p;
-        if (v0 > bv) { bv = v0; bi = i0; }
-        if (v1 > bv) { bv = v1; bi = i0 + 1; }
-        if (v2 > bv) { bv = v2; bi = i0 + 2; }
-        if (v3 > bv) { bv = v3; bi = i0 + 3; }
-      }
+      column_best<H>(z, (const float4*)(rslab + (size_t)c * rstride), ((uint32_t)(j * NC + c)) * n, bv, bi);
     }
     // the slab's best over its SEG lanes (xor offsets below SEG stay inside the segment)
 #pragma unroll
@@ -308,6 +313,78 @@ __global__ void __launch_bounds__(WARPS * 32, PER_SM) k_slab_cols(SlabArgs a) {
       if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
     }
     if (cl == 0 && live) a.cand[uslab] = make_float2(bv, __uint_as_float(bi));
+  }
+}
+
+// ── the slab a warp at a time, the next one on its way ──
+//
+// As k_slab_cols for 32 columns and one rden volume shared by every item, but a block walks a run of
+// slabs j-major with one staged tile of rden rows for all its warps, and the room that leaves in shared
+// memory gives each warp a slab of U: while a warp transforms one in registers, the copy of its next
+// is in flight. k_slab_cols holds its loads in the registers it computes in, so a warp either loads or
+// computes: 4.0 of 6.5 TB/s at L = 64, nc = 32, here 5.0, where instruction issue bounds it (some 3000
+// a slab of 16 KB, which alone allow 6.0). Items: before → now: 4096 1.09 → 0.87 ms, 1000 0.287 → 0.240,
+// 300 0.101 → 0.093, 16 0.024 → 0.022; L = 48, 1000 0.269 → 0.232.
+template <int H, int WARPS>
+struct StreamShared {
+  float rden[32][ColsRden<32, H>::RLD];
+  float2 slab[WARPS][H * 32];
+};
+
+template <int H, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, 1) k_slab_stream(SlabArgs a, long long chunk) {
+  constexpr int n = 2 * H, NC = 32;
+  extern __shared__ __align__(16) unsigned char stream_smem[];
+  StreamShared<H, WARPS>& s = *reinterpret_cast<StreamShared<H, WARPS>*>(stream_smem);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int L = a.d.L, nb = a.d.nb, ni = a.n_items;
+  const long long total = (long long)ni * nb;
+  long long t0 = blockIdx.x * chunk;
+  const long long t1 = t0 + chunk < total ? t0 + chunk : total;
+  float2* buf = s.slab[warp];
+  const uint32_t to = (uint32_t)__cvta_generic_to_shared(buf) + lane * 16;
+  while (t0 < t1) {
+    const int j = (int)(t0 / ni);
+    const long long first = (long long)j * ni;  // the slab of (j, item 0)
+    const long long te = first + ni < t1 ? first + ni : t1;
+    auto fetch = [&](long long t) {  // L rows of 256 bytes
+      const char* from = (const char*)(a.U + ((t - first) * nb + j) * L * NC) + lane * 16;
+#pragma unroll 8
+      for (int k = 0; k < L / 2; ++k)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + k * 512), "l"(from + k * 512) : "memory");
+      if ((L & 1) && lane < 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + (L / 2) * 512), "l"(from + (L / 2) * 512)
+                     : "memory");
+    };
+    long long t = t0 + warp;
+    if (t < te) fetch(t);
+    __syncthreads();  // every warp is done with the last j's rows
+    const float4* g = (const float4*)(a.rden + (size_t)j * NC * n);
+    for (int e = threadIdx.x; e < NC * n / 4; e += WARPS * 32) {
+      const int c = e / (n / 4), p4 = e - c * (n / 4);
+      *(float4*)(s.rden[c] + 4 * p4) = __ldg(g + e);
+    }
+    __syncthreads();
+    for (; t < te; t += WARPS) {
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      __syncwarp();
+      float2 z[H];
+#pragma unroll
+      for (int q = 0; q < H; ++q) z[q] = q < L ? buf[q * NC + lane] : make_float2(0.f, 0.f);
+      __syncwarp();
+      if (t + WARPS < te) fetch(t + WARPS);
+      float bv = -3.4e38f;
+      uint32_t bi = 0xffffffffu;
+      column_best<H>(z, (const float4*)s.rden[lane], (uint32_t)(j * NC + lane) * n, bv, bi);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
+        const uint32_t oi = __shfl_xor_sync(0xffffffffu, bi, o);
+        if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
+      }
+      if (lane == 0) a.cand[(t - first) * nb + j] = make_float2(bv, __uint_as_float(bi));
+    }
+    t0 = te;
   }
 }
 
@@ -676,6 +753,16 @@ static int slab_launch(const float* U, int n_items, const zeb_so3_dims_t* d, con
     }                                                                                                         \
     return zeb_launch_check("correlate slab (columns)");                                                    \
   }
+    // one rden volume for every item: the streaming walk, faster than k_slab_cols or level with it from
+    // 1 item up (its copies are of 16 bytes, so that U on an 8-byte boundary stays with k_slab_cols)
+    if (NC == 32 && H == 64 && a.rden_div >= n_items && ((uintptr_t)U & 15) == 0) {
+      constexpr int W = 12;
+      const long long chunk = (blocks + sms - 1) / sms;
+      const size_t sm = sizeof(StreamShared<64, W>);
+      cudaFuncSetAttribute(k_slab_stream<64, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+      k_slab_stream<64, W><<<(unsigned)((blocks + chunk - 1) / chunk), W * 32, sm, st>>>(a, chunk);
+      return zeb_launch_check("correlate slab (streamed)");
+    }
     ZEB_SLAB_COLS(8, 16, 4, 6)
     ZEB_SLAB_COLS(16, 16, 4, 6)
     ZEB_SLAB_COLS(16, 32, 4, 4)
