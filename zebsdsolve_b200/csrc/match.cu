@@ -603,7 +603,7 @@ extern "C" int zeb_dict_sims(const zeb_frame_t* fr, const float* vpair, int side
   a.q = (const float4*)dict_q;
   a.out = out;
   const size_t smem = (size_t)hw * 4;
-  if (smem > 48 * 1024) cudaFuncSetAttribute(k_dict_sims, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (smem > 40 * 1024) cudaFuncSetAttribute(k_dict_sims, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   k_dict_sims<<<n, 256, smem, (cudaStream_t)stream>>>(a);
   return zeb_launch_check("dict_sims");
 }

@@ -758,17 +758,18 @@ static int prep_launch(const void* raw, int pixel, int n, int src_h, int src_w, 
     // the tables take the place of the partial sums in the caller's scratch, whose size stays what it was:
     // one pattern of a large detector may not have the room
     if (d.table_floats(h, w) <= a.scratch_per * n && wsm <= 200 * 1024 && tsm <= 200 * 1024 && ((uintptr_t)scratch & 15) == 0) {
-      if (tsm > 48 * 1024) cudaFuncSetAttribute(k_wide_tables, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm);
+      // (the most either may ask for, whatever this call does: 48 KB beside a static array is already over)
+      cudaFuncSetAttribute(k_wide_tables, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
       k_wide_tables<<<h, 256, tsm, (cudaStream_t)stream>>>(a, a.scratch);
       int rc = zeb_launch_check("prep (wide blur tables)");
       if (rc) return rc;
-      if (wsm > 48 * 1024) cudaFuncSetAttribute(k_prep_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wsm);
+      cudaFuncSetAttribute(k_prep_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
       k_prep_wide<<<n, 256, wsm, (cudaStream_t)stream>>>(a, a.scratch, in ? 1 : 0);
       return zeb_launch_check("prep (wide blur)");
     }
   }
   size_t smem = a.use_smem ? 2 * (size_t)h * w * 4 : 0;
-  if (smem > 48 * 1024) cudaFuncSetAttribute(k_prep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (smem > 40 * 1024) cudaFuncSetAttribute(k_prep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   k_prep<<<n, 256, smem, (cudaStream_t)stream>>>(a);
   return zeb_launch_check("prep");
 }
