@@ -1,10 +1,12 @@
 """The correlation's transform along a with the next slab on its way (k_slab_stream: 32 columns of 64 points
 to a slab, one denominator volume) against the kernel that holds its loads in registers (k_slab_cols, which
-U on an 8-byte boundary takes): the same arithmetic in the same order, so the same bits (GPU only).
+U on an 8-byte boundary takes): the same arithmetic in the same order, so the same bits; 64 columns against
+the float64 transform, as test_gpu_slab_split has it (GPU only).
 """
 import ctypes
 
 import pytest
+import test_gpu_slab_split as split
 
 torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
@@ -43,3 +45,8 @@ def test_streamed_slabs_give_the_same_peaks(L, n):
         got.append((peaks, scratch[: n * 65 * 8].clone()))
     assert torch.equal(got[0][1], got[1][1])
     assert torch.equal(got[0][0], got[1][0])
+
+
+@pytest.mark.parametrize("L,n", [(64, 1), (33, 30), (63, 13), (48, 40)])
+def test_sixty_four_columns(L, n):
+    split.test_split_transform_finds_the_volume_s_largest_value(L, 2, n, 1 << 30)

@@ -318,24 +318,25 @@ __global__ void __launch_bounds__(WARPS * 32, PER_SM) k_slab_cols(SlabArgs a) {
 
 // ── the slab a warp at a time, the next one on its way ──
 //
-// As k_slab_cols for 32 columns and one rden volume shared by every item, but a block walks a run of
+// As k_slab_cols for 32 or 64 columns and one rden volume shared by every item, but a block walks a run of
 // slabs j-major with one staged tile of rden rows for all its warps, and the room that leaves in shared
-// memory gives each warp a slab of U: while a warp transforms one in registers, the copy of its next
+// memory gives each warp 32 columns of U: while a warp transforms them in registers, the copy of its next
 // is in flight. k_slab_cols holds its loads in the registers it computes in, so a warp either loads or
 // computes: 4.0 of 6.5 TB/s at L = 64, nc = 32, here 5.0, where instruction issue bounds it (some 3000
 // a slab of 16 KB, which alone allow 6.0). Items: before → now: 4096 1.09 → 0.87 ms, 1000 0.287 → 0.240,
-// 300 0.101 → 0.093, 16 0.024 → 0.022; L = 48, 1000 0.269 → 0.232.
-template <int H, int WARPS>
+// 300 0.101 → 0.093, 16 0.024 → 0.022; L = 48, 1000 0.269 → 0.232; L = 64 and nc = 64 (k_slab_split), 2048
+// 1.235 → 0.907; L = 48, 300 0.196 → 0.158.
+template <int NC, int H, int WARPS>
 struct StreamShared {
-  float rden[32][ColsRden<32, H>::RLD];
+  float rden[NC][ColsRden<NC, H>::RLD];
   float2 slab[WARPS][H * 32];
 };
 
-template <int H, int WARPS>
+template <int NC, int H, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, 1) k_slab_stream(SlabArgs a, long long chunk) {
-  constexpr int n = 2 * H, NC = 32;
+  constexpr int n = 2 * H;
   extern __shared__ __align__(16) unsigned char stream_smem[];
-  StreamShared<H, WARPS>& s = *reinterpret_cast<StreamShared<H, WARPS>*>(stream_smem);
+  StreamShared<NC, H, WARPS>& s = *reinterpret_cast<StreamShared<NC, H, WARPS>*>(stream_smem);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int L = a.d.L, nb = a.d.nb, ni = a.n_items;
   const long long total = (long long)ni * nb;
@@ -347,17 +348,18 @@ __global__ void __launch_bounds__(WARPS * 32, 1) k_slab_stream(SlabArgs a, long 
     const int j = (int)(t0 / ni);
     const long long first = (long long)j * ni;  // the slab of (j, item 0)
     const long long te = first + ni < t1 ? first + ni : t1;
-    auto fetch = [&](long long t) {  // L rows of 256 bytes
-      const char* from = (const char*)(a.U + ((t - first) * nb + j) * L * NC) + lane * 16;
+    // 32 columns, h·32 …, of a slab: L rows of 256 bytes, two an instruction
+    auto fetch = [&](long long t, int h) {
+      const char* from = (const char*)(a.U + (((t - first) * nb + j) * L + (lane >> 4)) * NC + h * 32) + (lane & 15) * 16;
 #pragma unroll 8
       for (int k = 0; k < L / 2; ++k)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + k * 512), "l"(from + k * 512) : "memory");
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + k * 512), "l"(from + k * (16 * NC)) : "memory");
       if ((L & 1) && lane < 16)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + (L / 2) * 512), "l"(from + (L / 2) * 512)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + (L / 2) * 512), "l"(from + (L / 2) * (16 * NC))
                      : "memory");
     };
     long long t = t0 + warp;
-    if (t < te) fetch(t);
+    if (t < te) fetch(t, 0);
     __syncthreads();  // every warp is done with the last j's rows
     const float4* g = (const float4*)(a.rden + (size_t)j * NC * n);
     for (int e = threadIdx.x; e < NC * n / 4; e += WARPS * 32) {
@@ -366,16 +368,20 @@ __global__ void __launch_bounds__(WARPS * 32, 1) k_slab_stream(SlabArgs a, long 
     }
     __syncthreads();
     for (; t < te; t += WARPS) {
-      asm volatile("cp.async.wait_all;" ::: "memory");
-      __syncwarp();
-      float2 z[H];
-#pragma unroll
-      for (int q = 0; q < H; ++q) z[q] = q < L ? buf[q * NC + lane] : make_float2(0.f, 0.f);
-      __syncwarp();
-      if (t + WARPS < te) fetch(t + WARPS);
       float bv = -3.4e38f;
       uint32_t bi = 0xffffffffu;
-      column_best<H>(z, (const float4*)s.rden[lane], (uint32_t)(j * NC + lane) * n, bv, bi);
+#pragma unroll 1
+      for (int h = 0; h < NC / 32; ++h) {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncwarp();
+        float2 z[H];
+#pragma unroll
+        for (int q = 0; q < H; ++q) z[q] = q < L ? buf[q * 32 + lane] : make_float2(0.f, 0.f);
+        __syncwarp();
+        if (h + 1 < NC / 32) fetch(t, h + 1);
+        else if (t + WARPS < te) fetch(t + WARPS, 0);
+        column_best<H>(z, (const float4*)s.rden[h * 32 + lane], (uint32_t)(j * NC + h * 32 + lane) * n, bv, bi);
+      }
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
         const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
@@ -753,16 +759,21 @@ static int slab_launch(const float* U, int n_items, const zeb_so3_dims_t* d, con
     }                                                                                                         \
     return zeb_launch_check("correlate slab (columns)");                                                    \
   }
-    // one rden volume for every item: the streaming walk, faster than k_slab_cols or level with it from
-    // 1 item up (its copies are of 16 bytes, so that U on an 8-byte boundary stays with k_slab_cols)
-    if (NC == 32 && H == 64 && a.rden_div >= n_items && ((uintptr_t)U & 15) == 0) {
-      constexpr int W = 12;
-      const long long chunk = (blocks + sms - 1) / sms;
-      const size_t sm = sizeof(StreamShared<64, W>);
-      cudaFuncSetAttribute(k_slab_stream<64, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-      k_slab_stream<64, W><<<(unsigned)((blocks + chunk - 1) / chunk), W * 32, sm, st>>>(a, chunk);
-      return zeb_launch_check("correlate slab (streamed)");
-    }
+    // One rden volume for every item: the streaming walk, faster than k_slab_cols (nc = 32) or k_slab_split
+    // (64; 8 items 0.028 → 0.029 ms, 100 0.090 → 0.083) or level with them from 1 item up. Not nc = 128,
+    // whose tile of rden rows takes a block too long for few items (5: 0.029 → 0.058). Its copies are of 16
+    // bytes, so that U on an 8-byte boundary stays with the others.
+#define ZEB_SLAB_STREAM(nc_, w_)                                                                             \
+  if (NC == nc_ && H == 64 && a.rden_div >= n_items && ((uintptr_t)U & 15) == 0) {                           \
+    const long long chunk = (blocks + sms - 1) / sms;                                                         \
+    const size_t sm = sizeof(StreamShared<nc_, 64, w_>);                                                      \
+    cudaFuncSetAttribute(k_slab_stream<nc_, 64, w_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);    \
+    k_slab_stream<nc_, 64, w_><<<(unsigned)((blocks + chunk - 1) / chunk), (w_)*32, sm, st>>>(a, chunk);       \
+    return zeb_launch_check("correlate slab (streamed)");                                                     \
+  }
+    ZEB_SLAB_STREAM(32, 12)
+    ZEB_SLAB_STREAM(64, 12)
+#undef ZEB_SLAB_STREAM
     ZEB_SLAB_COLS(8, 16, 4, 6)
     ZEB_SLAB_COLS(16, 16, 4, 6)
     ZEB_SLAB_COLS(16, 32, 4, 4)
@@ -773,7 +784,8 @@ static int slab_launch(const float* U, int n_items, const zeb_so3_dims_t* d, con
     // Longer columns, and more columns than a warp's share of shared memory stages, take the block-wide
     // split; measured on both sides of each line (items: before → split): L = 128, nc = 64 (256): 10.17
     // → 0.70 ms; L = 80, nc = 128 (128): 9.47 → 0.59; L = 64, nc = 128 (1024): 19.7 → 1.23; L = 64, nc = 64
-    // (2048): 1.99 (k_slab_cols) → 1.23; but nc = 32 (4096): 1.10 against 1.25, and stays with k_slab_cols.
+    // (2048, U on an 8-byte boundary): 1.99 (k_slab_cols) → 1.23; but nc = 32 (4096): 1.10 against 1.25, and
+    // stays with k_slab_cols.
     if (H == 128 && NC % 32 == 0) return split_launch<16, 8, 3>(a, sms, st);
     if (H == 64 && NC % 32 == 0) return split_launch<8, 8, 4>(a, sms, st);
   }
