@@ -221,21 +221,6 @@ int zeb_tc_pack_master(const zeb_so3_dims_t* d, int split, const double* Y, void
 size_t zeb_tc_master_bytes(const zeb_so3_dims_t* d, int split);
 size_t zeb_tc_patterns_bytes(const zeb_so3_dims_t* d, int split, int n_items);
 
-/* The FP32 form's spectrum on the tensor cores: zeb_spectrum_f32's U, at its accuracy against 64 bits or
- * better, from operands split x = hi + lo into two FP16 values (lo*hi + hi*lo + hi*hi, FP32
- * accumulation in tensor memory from the highest degree down). 24 <= L <= 128. A is the master's
- * table packed once per phase by zeb_x2_pack_master from the FP64 Y of zeb_correlation_table
- * (zeb_x2_master_bytes bytes), times `scale`, a power of two with scale * max|Re Y|, |Im Y| <= 16384; the
- * same scale goes to zeb_spectrum_x2. alm: coefficients of at most unit norm
- * (zeb_sphere_coefficients with ZEB_FLAG_NORM). B is scratch of zeb_x2_patterns_bytes bytes that the
- * call packs from alm; status as zeb_spectrum_bf16. Replaces Spherical.spectrum
- * (src/spherical.zig:369-382; shaders/so3.wgsl spectrum). */
-size_t zeb_x2_master_bytes(const zeb_so3_dims_t* d); /* 0: dims it does not take */
-size_t zeb_x2_patterns_bytes(const zeb_so3_dims_t* d, int n_items);
-int zeb_x2_pack_master(const zeb_so3_dims_t* d, const double* Y, float scale, void* A, void* stream);
-int zeb_spectrum_x2(const float* alm, int n_items, const zeb_so3_dims_t* d, const void* A, float scale, void* B,
-                    float* U, int* status, void* stream);
-
 /* The BF16 form's spectrum kept in FP16 (half the bytes of U): zeb_spectrum_bf16's GEMM, its
  * accumulators scaled by `scale` and rounded to FP16 as they drain, stored as
  * U16[item / 128][j·nc + c][m'][re|im][item % 128] with the items padded to a multiple of 128

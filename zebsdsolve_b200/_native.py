@@ -68,10 +68,6 @@ _SIGS = {
     "zeb_tc_pack_master": ([ctypes.POINTER(So3Dims), c_int, P, P, P], c_int),
     "zeb_tc_master_bytes": ([ctypes.POINTER(So3Dims), c_int], c_size_t),
     "zeb_tc_patterns_bytes": ([ctypes.POINTER(So3Dims), c_int, c_int], c_size_t),
-    "zeb_x2_master_bytes": ([ctypes.POINTER(So3Dims)], c_size_t),
-    "zeb_x2_patterns_bytes": ([ctypes.POINTER(So3Dims), c_int], c_size_t),
-    "zeb_x2_pack_master": ([ctypes.POINTER(So3Dims), P, c_float, P, P], c_int),
-    "zeb_spectrum_x2": ([P, c_int, ctypes.POINTER(So3Dims), P, c_float, P, P, P, P], c_int),
     "zeb_peaks_scratch_bytes": ([ctypes.POINTER(So3Dims), c_int], c_size_t),
     "zeb_correlate_peaks": ([P, c_int, ctypes.POINTER(So3Dims), P, P, c_int, P, P, P], c_int),
     "zeb_spectrum_h_bytes": ([ctypes.POINTER(So3Dims), c_int], c_size_t),
@@ -126,7 +122,7 @@ ZEB_SETTLE6_STATE = 44
 
 # kernels each entry point launches (for the launch counts the benchmark reports)
 KERNELS = {"zeb_nlpar": 5, "zeb_pc_splat": 0, "zeb_sums6_list": 1, "zeb_clahe": 4, "zeb_combine": 1, "zeb_master_symmetrize": 1, "zeb_prep": 1, "zeb_prep_ex": 1, "zeb_prep_reduced": 1, "zeb_sphere_coefficients": 3, "zeb_sphere_coefficients_spans": 3, "zeb_sphere_spans": 1, "zeb_spectrum_f32": 1,
-           "zeb_spectrum_bf16": 2, "zeb_tc_pack_master": 0, "zeb_x2_pack_master": 0, "zeb_spectrum_x2": 2, "zeb_correlate_peaks": 2, "zeb_correlate_peaks_static": 2, "zeb_spectrum_bf16_h": 2, "zeb_correlate_peaks_h": 2, "zeb_master_quads": 1, "zeb_refine_list_h": 1, "zeb_pack_panel_split": 1, "zeb_project_bf16": 1, "zeb_project_f32": 1, "zeb_correlate_volume": 1, "zeb_rden_build": 1,
+           "zeb_spectrum_bf16": 2, "zeb_tc_pack_master": 0, "zeb_correlate_peaks": 2, "zeb_correlate_peaks_static": 2, "zeb_spectrum_bf16_h": 2, "zeb_correlate_peaks_h": 2, "zeb_master_quads": 1, "zeb_refine_list_h": 1, "zeb_pack_panel_split": 1, "zeb_project_bf16": 1, "zeb_project_f32": 1, "zeb_correlate_volume": 1, "zeb_rden_build": 1,
            "zeb_refine": 1, "zeb_chance": 1, "zeb_project": 1, "zeb_records_fz": 1, "zeb_records_fz_bunge": 1, "zeb_det6": 1, "zeb_det6_list": 1, "zeb_solve6": 1, "zeb_settle6": 1, "zeb_pack_panel": 1, "zeb_mask_list": 1, "zeb_refine_list": 1, "zeb_dict_sims": 1, "zeb_match_bf16": 1, "zeb_match_f32": 1, "zeb_match_best": 1, "zeb_master_blur_pass": 1, "zeb_master_gradient": 1, "zeb_master_pairs": 1,
            "zeb_master_sample_grid": 1, "zeb_gauss_legendre": 1, "zeb_legendre_table": 1, "zeb_wigner_half_pi": 1,
            "zeb_correlation_table": 1}

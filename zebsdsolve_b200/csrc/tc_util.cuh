@@ -177,27 +177,6 @@ __device__ __forceinline__ uint64_t umma_desc_mn(uint32_t saddr, uint32_t lbo, u
   d |= (uint64_t)2 << 61;
   return d;
 }
-// A drain's stores. A warp holds 32 accumulator rows (lane = row); its values go through a buffer of its
-// own in shared memory so that each store instruction writes whole 128-byte lines, 512 bytes in all
-// (such stores from four warps an SM reach 6.3 TB/s on a B200 whatever the distance between the lines),
-// and no warp waits for another.
-//
-// 32 rows × 32 patterns of FP32 (v[c]: pattern c): dst + p·stride is where lane's four rows of pattern p go
-__device__ __forceinline__ void drain_f32(float* buf, int lane, const uint32_t (&v)[32], float scale, float* dst,
-                                          size_t stride, int patterns) {
-  __syncwarp();  // the last chunk has been read out of buf
-#pragma unroll
-  for (int c = 0; c < 32; ++c) buf[c * 32 + lane] = __uint_as_float(v[c]) * scale;
-  __syncwarp();
-  const float4* src = (const float4*)buf + lane;
-  float* d = dst + (size_t)(lane >> 3) * stride;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const float4 x = src[i * 32];
-    if (4 * i + (lane >> 3) < patterns) *(float4*)d = x;
-    d += 4 * stride;
-  }
-}
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_read1() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }

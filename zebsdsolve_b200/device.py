@@ -179,16 +179,6 @@ class PhaseBand:
             self.A = torch.empty(nbytes, dtype=torch.uint8, device=dev)
             N.call("zeb_tc_pack_master", ctypes.byref(self.dims), self.split, ptr(torch.view_as_real(Y64)),
                    ptr(self.A), stream_ptr())
-        # the FP32 form: the table split into FP16 pairs for the tensor cores (zeb_spectrum_x2), where
-        # the bandwidth is one it takes (elsewhere zeb_spectrum_f32 reads Y_f)
-        self.x2_scale = None
-        nbytes = N.load().zeb_x2_master_bytes(ctypes.byref(self.dims)) if precision == "f32" else 0
-        if nbytes:
-            top = float(torch.view_as_real(Y64).abs().max())
-            self.x2_scale = 2.0 ** math.floor(math.log2(16384.0 / max(top, 1e-30)))
-            self.A = torch.empty(nbytes, dtype=torch.uint8, device=dev)
-            N.call("zeb_x2_pack_master", ctypes.byref(self.dims), ptr(torch.view_as_real(Y64)), self.x2_scale,
-                   ptr(self.A), stream_ptr())
         # the BF16 form keeps the spectrum in FP16 (zeb_spectrum_bf16_h, zeb_correlate_peaks_h) where
         # the tensor-core transform along a takes the bandwidth; bf16x3 keeps FP32 (its point is
         # FP32-quality U)

@@ -174,7 +174,6 @@ class Engine:
         self._full = False  # at_full: the stored size is the level being worked at
         self._resident = None  # the scan's filtered patterns a whole pass kept on the device (prepared)
         self._whole_pass = False  # an indexing run over the scan is under way (its batches are kept)
-        self._region_few = False  # the indexing run's region has a few cells (plain_spectrum)
         self.geo_given = Geometry()  # the geometry as given (set_geometry), where a full fit starts
         self._nl_view = None  # what averaging with neighbours did to the last pattern looked at
         self._nl_report = False  # log what the averaging did to the next batch (an indexing run's first)
@@ -564,27 +563,10 @@ class Engine:
             ph.rden = rden
             ph.rden_key = key
 
-    # A run over no more cells than this (a look at single patterns) and a run without refinement keep the
-    # plain FP32 spectrum. Every pattern of a phase with a two-fold axis across z has pairs of peaks that
-    # are equal but for rounding; refined, either leads to the same orientation, but the peak itself is an
-    # unrefined run's result, and a single look's record should not move with the arithmetic. 16 patterns
-    # at L = 64 take 77 µs so against 51, of a 1.9 ms call; 4096 at L = 32, unrefined, 0.47 ms against 0.25 of 3.0.
-    FEW_CELLS = 64
-
-    def plain_spectrum(self, n):
-        """Whether a run over n cells keeps the plain FP32 spectrum (precision "f32"): an indexing run
-        goes by its whole region, however its cells are cut into steps, sweeps or ranks' shares."""
-        few = self._region_few if self._whole_pass else n <= self.FEW_CELLS
-        return few or not self.set["refine"]
-
-    def spectrum(self, alm, n, ph, Y, U, tensor_cores=True, plain=False):
-        """spherical.zig:369-382 — U of n items: on the tensor cores when the phase has its packed
-        table (the FP32 form's in FP16 pairs, unless `plain`; the BF16 forms'), else in plain FP32."""
-        if tensor_cores and not plain and ph.x2_scale is not None and Y is ph.Y_f:
-            B = self.buf("tc_b", N.load().zeb_x2_patterns_bytes(ctypes.byref(ph.dims), n), torch.uint8)
-            N.call("zeb_spectrum_x2", ptr(alm), n, ctypes.byref(ph.dims), ptr(ph.A), ph.x2_scale, ptr(B), ptr(U),
-                   ptr(self.tc_status()), stream_ptr())
-        elif tensor_cores and ph.split is not None and Y is ph.Y_f:
+    def spectrum(self, alm, n, ph, Y, U, tensor_cores=True):
+        """spherical.zig:369-382 — U of n items: on the tensor cores (BF16 form) when the phase
+        has its packed table, else in plain FP32."""
+        if tensor_cores and ph.A is not None and Y is ph.Y_f:
             B = self.buf("tc_b", N.load().zeb_tc_patterns_bytes(ctypes.byref(ph.dims), ph.split, n), torch.uint8)
             N.call("zeb_spectrum_bf16", ptr(alm), n, ctypes.byref(ph.dims), ph.split, ptr(ph.A), ptr(B), ptr(U),
                    ptr(self.tc_status()), stream_ptr())
@@ -1094,12 +1076,11 @@ class Engine:
         self._spans[key] = sp
         return sp
 
-    def run_device(self, raw, cells, bandwidth=None, timer=None, method="spherical", grid=None, pre=None, plain=False):
+    def run_device(self, raw, cells, bandwidth=None, timer=None, method="spherical", grid=None, pre=None):
         """One pass of the device path over n = len(cells) stored patterns already on the device:
         records [phase][cell][8] as a device tensor (engine.zig:2005-2122, no readback). pre: the
         cells' items already on the device with their bounding box (items_of's two results), as
-        index_pipelined copies them ahead of the pass's patterns. plain: the FP32 form's
-        spectrum in plain FP32 (plain_spectrum)."""
+        index_pipelined copies them ahead of the pass's patterns."""
         self.counts["submits"] += 1
         if method != "spherical":
             return self.run_device_dictionary(raw, cells, method, int(grid or self.set["dict_grid"]), timer)
@@ -1150,7 +1131,7 @@ class Engine:
                     continue
                 U = self.buf("spec", N.load().zeb_spectrum_bytes(ctypes.byref(ph.dims), nt) // 4 + 1)
                 mark("spectrum")
-                self.spectrum(a0, nt, ph, ph.Y_f, U, plain=plain)
+                self.spectrum(a0, nt, ph, ph.Y_f, U)
                 mark("peaks")
                 N.call("zeb_correlate_peaks", ptr(U), nt, ctypes.byref(ph.dims), ptr(bt.tw), ptr(ph.rden), 1 << 30,
                        ptr(peaks[t0 * 8:]), ptr(cand), stream_ptr())
@@ -1447,7 +1428,7 @@ class Engine:
         rows, cols, h, w = self.info()
         raw = self.buf("raw_up", n * h * w, self.raw_dtype()).view(-1)[: n * h * w].view(n, h, w)
         self.upload_raw(cells, raw, torch.cuda.current_stream())
-        recs = self.run_device(raw, cells, bandwidth, method=method, grid=grid, plain=self.plain_spectrum(n))
+        recs = self.run_device(raw, cells, bandwidth, method=method, grid=grid)
         fzd, bgd = self.fz_of(recs)
         self._last_fz = (fzd.cpu().numpy(), bgd.cpu().numpy())
         out = recs.cpu().numpy()
@@ -1542,7 +1523,6 @@ class Engine:
         if len(cells) == 0:
             return
         self.prepare(bandwidth, method, grid)
-        plain = self.plain_spectrum(len(cells))
         rows, cols, h, w = self.info()
         B = min(self.device_batch(), len(cells))
         comp = torch.cuda.current_stream()
@@ -1603,7 +1583,7 @@ class Engine:
             k = i % 2
             comp.wait_event(up_done[k])
             cb = parts[i]
-            recs = self.run_device(raw[k][: len(cb)], cb, bandwidth, method=method, grid=grid, pre=pre[k], plain=plain)
+            recs = self.run_device(raw[k][: len(cb)], cb, bandwidth, method=method, grid=grid, pre=pre[k])
             ev = torch.cuda.Event()
             ev.record(comp)
             comp_done[k] = ev
@@ -1707,7 +1687,6 @@ class Engine:
         self.index_cells_list = cells
         self.index_done = 0
         self.index_region = len(cells)
-        self._region_few = len(cells) <= self.FEW_CELLS
         self.index_sweep = 0
         self.index_accepted = 0
         self.cancel = False

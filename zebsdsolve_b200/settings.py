@@ -62,9 +62,8 @@ DEFAULTS = dict([
     ("sweeps", 1), ("sweep_bandwidth", 32), ("sweep_dict_grid", 20), ("sweep_method", "same"),
     ("pca_components", 256), ("pca_epochs", 2),
     ("accept_nmi", 0.0), ("accept_z", 15.0), ("accept_step_deg", 0.2),
-    # this engine's own: which arithmetic the Wigner-d contraction runs in ("f32": FP32 quality,
-    # operands as FP16 pairs on the tensor cores for bandwidths 24 to 128, plain FP32 on the CUDA cores
-    # for others, for a few cells and without refinement; "bf16": BF16 tensor cores with FP32 accumulation, operands split
+    # this engine's own: which arithmetic the Wigner-d contraction runs in ("f32": the plain FP32
+    # form on the CUDA cores; "bf16": BF16 tensor cores with FP32 accumulation, operands split
     # hi + lo for the orders l <= 16; "bf16x3": split for every order, near FP32 throughout)
     ("precision", "f32"),
 ])
