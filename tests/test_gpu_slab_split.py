@@ -1,5 +1,6 @@
 """The correlation's transform along a where a block splits it over its warps (k_slab_split: columns of
-128 points, and 64-point columns of 64 or 128 to a slab), against a float64 inverse FFT (GPU only).
+128 points, and 64-point columns of 128 to a slab), against a float64 inverse FFT, and its values against the
+shared-memory transform's bits; 64-point columns of 64 to a slab against the FFT too (GPU only).
 
 Tolerance: a value is a sum of L terms f·V·e with Σ|f V| <= s, through log2(n) stages of single-precision
 butterflies: |error| <= 2 (log2 n + 2) 2^-24 s for its column's s, scaled by rden.
@@ -88,3 +89,35 @@ def test_split_transform_keeps_the_first_of_equal_values(L, fold):
     # first among 1's past the damped cells; first among the -0.5's (the largest of the negatives)
     assert abs(peaks[0, 4] - 1) < 1e-6 and np.allclose(peaks[0, 5:8], [3 * step, 0, 0], atol=0.51 * step)
     assert abs(peaks[1, 4] + 0.5) < 1e-6 and np.allclose(peaks[1, 6:8], 0, atol=1e-6) and peaks[1, 5] <= 0.51 * step
+
+
+@pytest.mark.parametrize("L,fold,n,div", [(128, 4, 5, 1 << 30), (65, 4, 6, 4), (80, 2, 3, 1), (92, 2, 2, 1 << 30),
+                                          (33, 1, 4, 3), (64, 1, 3, 1 << 30)])
+def test_split_transform_gives_the_shared_memory_transform_s_bits(L, fold, n, div):
+    """Every slab's candidate is the largest of zeb_correlate_volume's values (k_slab, the transform that a
+    slab of these sizes took before) times its denominators: the same stages with the same twiddles."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from zebsdsolve_b200 import _native as N
+
+    d = _dims(L, fold)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(L * 16 + fold)
+    U = torch.randn(n, d.nb, L, d.nc, 2, device="cuda", generator=g)
+    volumes = -(-n // min(div, n))
+    rden = torch.rand(volumes, d.nb, d.nc, d.n, device="cuda", generator=g) + 0.5
+    vol = torch.empty(n, d.nb, d.nc, d.n, device="cuda")
+    tw = _tw()
+    N.call("zeb_correlate_volume", _p(U), n, ctypes.byref(d), _p(tw), _p(vol), _sp())
+    want = (vol * rden[torch.arange(n, device="cuda") // min(div, n)]).reshape(n, d.nb, -1)
+    peaks = torch.zeros(n, 8, device="cuda")
+    scratch = torch.empty(N.load().zeb_peaks_scratch_bytes(ctypes.byref(d), n), dtype=torch.uint8, device="cuda")
+    N.call("zeb_correlate_peaks", _p(U), n, ctypes.byref(d), _p(tw), _p(rden), div, _p(peaks), _p(scratch), _sp())
+    key = scratch.view(torch.int32).view(n, d.nb, 2).cpu().numpy().view(np.uint32)
+    top = key[..., 1]
+    value = np.where(top >> 31 == 1, top ^ np.uint32(1 << 31), ~top).astype(np.uint32).view(np.float32)
+    index = (~key[..., 0]).astype(np.int64) - np.arange(d.nb) * d.nc * d.n
+    best = want.max(-1).values
+    assert np.array_equal(value, best.cpu().numpy())
+    at = want.gather(2, torch.as_tensor(index, device="cuda")[..., None])[..., 0]
+    assert torch.equal(at, best) and torch.equal(peaks[:, 4], best.max(1).values)

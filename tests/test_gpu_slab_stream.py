@@ -1,7 +1,7 @@
-"""The correlation's transform along a with the next slab on its way (k_slab_stream: 32 columns of 64 points
-to a slab, one denominator volume) against the kernel that holds its loads in registers (k_slab_cols, which
-U on an 8-byte boundary takes): the same arithmetic in the same order, so the same bits; 64 columns against
-the float64 transform, as test_gpu_slab_split has it (GPU only).
+"""The correlation's transform along a with the next slab on its way (k_slab_stream: 32 or 64 columns
+of 64 points to a slab, one denominator volume) against the kernel that holds its loads in
+registers (k_slab_cols, which U on an 8-byte boundary takes): the same arithmetic in the same order, so the same
+bits; 64 columns also against the float64 transform, as test_gpu_slab_split has it (GPU only).
 """
 import ctypes
 
@@ -16,19 +16,21 @@ def _p(t):
     return ctypes.c_void_p(t.data_ptr())
 
 
-@pytest.mark.parametrize("L,n", [(64, 1), (64, 13), (33, 200), (63, 77), (48, 300), (64, 700)])
-def test_streamed_slabs_give_the_same_peaks(L, n):
+@pytest.mark.parametrize("L,n,fold", [(64, 1, 4), (64, 13, 4), (33, 200, 4), (63, 77, 4), (48, 300, 4), (64, 700, 4),
+                                      (64, 40, 2), (35, 9, 2)])
+def test_streamed_slabs_give_the_same_peaks(L, n, fold):
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")
     from zebsdsolve_b200 import _native as N
 
-    d = N.So3Dims(L, 128, 65, 32, 4, (L - 1) // 4, L * (L + 1) // 2)
+    nc = 128 // fold
+    d = N.So3Dims(L, 128, 65, nc, fold, (L - 1) // fold, L * (L + 1) // 2)
     g = torch.Generator(device="cuda")
     g.manual_seed(L * 1000 + n)
-    count = n * 65 * L * 32 * 2
+    count = n * 65 * L * nc * 2
     both = torch.empty(count + 4, device="cuda")
     U = torch.randn(count, device="cuda", generator=g)
-    rden = torch.rand(65 * 32 * 128, device="cuda", generator=g) + 0.5
+    rden = torch.rand(65 * nc * 128, device="cuda", generator=g) + 0.5
     rden[::13] = 0
     t = -2j * torch.pi * torch.arange(1024, dtype=torch.float64) / 1024
     tw = torch.view_as_real(torch.exp(t).to(torch.complex64)).contiguous().cuda()

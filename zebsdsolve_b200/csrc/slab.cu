@@ -175,6 +175,71 @@ __device__ __forceinline__ void fft_reg(float2 (&x)[N]) {
   }
 }
 
+// The transform k_slab_split takes in two parts, in the bits of k_slab's: radix-2 stages with the table's
+// twiddles, each product fused as there (left to the compiler, a negative constant twiddle swaps the
+// rounded and the fused product).
+__device__ __forceinline__ float2 cmul_fixed(float2 b, float2 w) {
+  return make_float2(fmaf(b.x, w.x, -__fmul_rn(b.y, w.y)), fmaf(b.x, w.y, __fmul_rn(b.y, w.x)));
+}
+
+// its first log2(N) stages: an N-point transform, natural order in and out
+template <int N>
+__device__ __forceinline__ void fft_first(float2 (&x)[N]) {
+  constexpr int LG = log2_const(N);
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const int j = brev_bits(i, LG);
+    if (j > i) {
+      float2 t = x[i];
+      x[i] = x[j];
+      x[j] = t;
+    }
+  }
+#pragma unroll
+  for (int s = 1; s <= LG; ++s) {
+#pragma unroll
+    for (int e = 0; e < N / 2; ++e) {
+      const int h = 1 << (s - 1);
+      const int j = e & (h - 1);
+      const int i0 = ((e >> (s - 1)) << s) + j;
+      const float2 b = x[i0 + h];
+      const float2 t = j == 0 ? b : 2 * j == h ? make_float2(b.y, -b.x) : cmul_fixed(b, tw_of<N>(j * (N >> s)));
+      const float2 a = x[i0];
+      x[i0] = make_float2(a.x + t.x, a.y + t.y);
+      x[i0 + h] = make_float2(a.x - t.x, a.y - t.y);
+    }
+  }
+}
+
+// and the last log2(R2) stages of R1·R2 points: x[r] is point p1 of the R1-point transform of the residue r
+// modulo R2, and becomes point p1 + R1·i of the whole; tws: e^{−2πi t/(2 R1 R2)}
+template <int R1, int R2>
+__device__ __forceinline__ void fft_last(float2 (&x)[R2], int p1, const float2* tws) {
+  constexpr int LG = log2_const(R2);
+#pragma unroll
+  for (int i = 0; i < R2; ++i) {
+    const int j = brev_bits(i, LG);
+    if (j > i) {
+      float2 t = x[i];
+      x[i] = x[j];
+      x[j] = t;
+    }
+  }
+#pragma unroll
+  for (int s = 1; s <= LG; ++s) {
+#pragma unroll
+    for (int e = 0; e < R2 / 2; ++e) {
+      const int h = 1 << (s - 1);
+      const int j = e & (h - 1);
+      const int i0 = ((e >> (s - 1)) << s) + j;
+      const float2 t = cmul_fixed(x[i0 + h], tws[(p1 + R1 * j) * (R2 >> (s - 1))]);
+      const float2 a = x[i0];
+      x[i0] = make_float2(a.x + t.x, a.y + t.y);
+      x[i0 + h] = make_float2(a.x - t.x, a.y - t.y);
+    }
+  }
+}
+
 // a column's values from its coefficients z (0 beyond L) and row rd of rden: the largest kept in
 // (bv, bi), the first of equal ones (base: the column's first volume index)
 template <int H>
@@ -324,8 +389,8 @@ __global__ void __launch_bounds__(WARPS * 32, PER_SM) k_slab_cols(SlabArgs a) {
 // is in flight. k_slab_cols holds its loads in the registers it computes in, so a warp either loads or
 // computes: 4.0 of 6.5 TB/s at L = 64, nc = 32, here 5.0, where instruction issue bounds it (some 3000
 // a slab of 16 KB, which alone allow 6.0). Items: before → now: 4096 1.09 → 0.87 ms, 1000 0.287 → 0.240,
-// 300 0.101 → 0.093, 16 0.024 → 0.022; L = 48, 1000 0.269 → 0.232; L = 64 and nc = 64 (k_slab_split), 2048
-// 1.235 → 0.907; L = 48, 300 0.196 → 0.158.
+// 300 0.101 → 0.093, 16 0.024 → 0.022; L = 48, 1000 0.269 → 0.232; L = 64 and nc = 64, 512 0.536 → 0.278, 8
+// 0.041 → 0.038, 1 0.039 → 0.036.
 template <int NC, int H, int WARPS>
 struct StreamShared {
   float rden[NC][ColsRden<NC, H>::RLD];
@@ -398,15 +463,19 @@ __global__ void __launch_bounds__(WARPS * 32, 1) k_slab_stream(SlabArgs a, long 
 //
 // Where a column's half-length transform (H points) does not fit one lane's registers, or nc columns
 // of rden rows do not fit a warp's share of shared memory, a block of R2/2 warps takes 32 columns of a
-// slab (lane = column) and computes H = R1·R2 in two steps: warp w holds the rows of the residues
+// slab (lane = column) and computes H = R1·R2 in two parts: warp w holds the rows of the residues
 // (w, R2 − w) modulo R2 (warp 0: 0 and R2/2), which the real transform's pairs (q, H − q) close over,
-// so that Z is formed in registers from loads that are all in flight at once; R1-point transforms,
-// twiddles, one exchange through shared memory, R2-point transforms. The 32 columns' rden rows stay in
+// so that Z is formed in registers from loads that are all in flight at once; the first log2(R1) stages,
+// one exchange through shared memory, the last log2(R2). The 32 columns' rden rows stay in
 // shared memory while the block walks a run of items of one j. Each item's largest value is reduced
 // over the block first and its index looked for only in the warps that hold it. A slab of more than
 // 32 columns has several blocks: its candidate is a 64-bit key (the value, order-preserving; then the
 // lowest index), combined by atomicMax over zeroed scratch.
-// Bound by the loads' latency and issue together: U is read once, at 3.1 (H = 128) to 3.5 TB/s (H = 64)
+// Every value is k_slab's bit for bit: the same radix-2 butterflies with the same twiddles. (The usual
+// split, twiddles before transforms of R2 points with constants, has fewer products and ran 3 to 6 %
+// faster, but its rounding moved refined results of L = 128 by 2e-4 of their size: an orientation's
+// move puts pixels into other bins of the NMI.)
+// Bound by the loads' latency and issue together: U is read once, at 2.9 (H = 128) to 3.5 TB/s (H = 64)
 // of 6.5 measured; the shared-memory transform it takes over from (k_slab) ran at 0.2 TB/s, every
 // radix-2 stage a trip through shared memory between block barriers.
 struct SplitKey {
@@ -476,7 +545,7 @@ __global__ void __launch_bounds__(R2 * 16, PER_SM) k_slab_split(SlabArgs a, int 
     auto pair = [&](float2& xq, float2& xm, int q) {
       const float2 w = tws[q];
       const float2 sm = make_float2(xq.x + xm.x, xq.y - xm.y), df = make_float2(xq.x - xm.x, xq.y + xm.y);
-      const float2 t = make_float2(w.x * df.x - w.y * df.y, w.x * df.y + w.y * df.x);
+      const float2 t = make_float2(fmaf(w.x, df.x, -__fmul_rn(w.y, df.y)), fmaf(w.x, df.y, __fmul_rn(w.y, df.x)));
       xq = make_float2(sm.x - t.y, sm.y + t.x);
       xm = make_float2(sm.x + t.y, t.x - sm.y);
     };
@@ -492,14 +561,10 @@ __global__ void __launch_bounds__(R2 * 16, PER_SM) k_slab_split(SlabArgs a, int 
 #pragma unroll
       for (int k = 0; k < R1; ++k) pair(xa[k], xb[R1 - 1 - k], ra + R2 * k);
     }
-    fft_reg<R1>(xa);
-    fft_reg<R1>(xb);
+    fft_first<R1>(xa);
+    fft_first<R1>(xb);
 #pragma unroll
     for (int k = 0; k < R1; ++k) {
-      if (k > 0) {
-        xa[k] = cmulf(xa[k], tws[2 * ra * k]);
-        xb[k] = cmulf(xb[k], tws[(2 * rb * k) & (N - 1)]);
-      }
       ex[(ra * R1 + k) * 32 + lane] = xa[k];
       ex[(rb * R1 + k) * 32 + lane] = xb[k];
     }
@@ -511,7 +576,7 @@ __global__ void __launch_bounds__(R2 * 16, PER_SM) k_slab_split(SlabArgs a, int 
       const int p1 = warp * G + g;
 #pragma unroll
       for (int q2 = 0; q2 < R2; ++q2) z[g][q2] = ex[(q2 * R1 + p1) * 32 + lane];
-      fft_reg<R2>(z[g]);
+      fft_last<R1, R2>(z[g], p1, tws);
 #pragma unroll
       for (int p2 = 0; p2 < R2; ++p2) {
         const float2 r = *(const float2*)(rt + lane * S::RLD + 2 * (p1 + R1 * p2));
@@ -759,10 +824,10 @@ static int slab_launch(const float* U, int n_items, const zeb_so3_dims_t* d, con
     }                                                                                                         \
     return zeb_launch_check("correlate slab (columns)");                                                    \
   }
-    // One rden volume for every item: the streaming walk, faster than k_slab_cols (nc = 32) or k_slab_split
-    // (64; 8 items 0.028 → 0.029 ms, 100 0.090 → 0.083) or level with them from 1 item up. Not nc = 128,
-    // whose tile of rden rows takes a block too long for few items (5: 0.029 → 0.058). Its copies are of 16
-    // bytes, so that U on an 8-byte boundary stays with the others.
+    // One rden volume for every item: the streaming walk, faster than k_slab_cols from 1 item up (nc = 64:
+    // 1 item 0.039 → 0.036 ms, 512 0.536 → 0.278). Not nc = 128, whose tile of rden rows takes a block too
+    // long for few items (5: 0.029 → 0.058). Its copies are of 16 bytes, so that U on an 8-byte boundary
+    // stays with the others.
 #define ZEB_SLAB_STREAM(nc_, w_)                                                                             \
   if (NC == nc_ && H == 64 && a.rden_div >= n_items && ((uintptr_t)U & 15) == 0) {                           \
     const long long chunk = (blocks + sms - 1) / sms;                                                         \
@@ -780,14 +845,14 @@ static int slab_launch(const float* U, int n_items, const zeb_so3_dims_t* d, con
     ZEB_SLAB_COLS(32, 32, 4, 4)
     ZEB_SLAB_COLS(64, 32, 4, 4)
     ZEB_SLAB_COLS(32, 64, 4, 3)
+    ZEB_SLAB_COLS(64, 64, 4, 3)
 #undef ZEB_SLAB_COLS
     // Longer columns, and more columns than a warp's share of shared memory stages, take the block-wide
-    // split; measured on both sides of each line (items: before → split): L = 128, nc = 64 (256): 10.17
-    // → 0.70 ms; L = 80, nc = 128 (128): 9.47 → 0.59; L = 64, nc = 128 (1024): 19.7 → 1.23; L = 64, nc = 64
-    // (2048, U on an 8-byte boundary): 1.99 (k_slab_cols) → 1.23; but nc = 32 (4096): 1.10 against 1.25, and
-    // stays with k_slab_cols.
+    // split; items: k_slab → split: L = 128, nc = 64: 256 10.11 → 0.75 ms, 1 0.087 → 0.036; L = 80, nc = 128:
+    // 128 9.45 → 0.61, 1 0.131 → 0.043; L = 64, nc = 128: 512 9.68 → 0.63, 1 0.085 → 0.031. Not fewer columns
+    // of 64 points (nc = 32, 4096: 1.10 → 1.25).
     if (H == 128 && NC % 32 == 0) return split_launch<16, 8, 3>(a, sms, st);
-    if (H == 64 && NC % 32 == 0) return split_launch<8, 8, 4>(a, sms, st);
+    if (H == 64 && NC == 128) return split_launch<8, 8, 4>(a, sms, st);
   }
   if (vol) {
     cudaFuncSetAttribute(k_slab<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -935,7 +1000,7 @@ extern "C" int zeb_correlate_peaks_static(const float* U, int n_items, const zeb
       g_static_next = (g_static_next + 1) % 64;
     }
   }
-  // every slab writes its candidate before k_peak_finish reads it: nothing needs clearing
+  // every slab writes its candidate, or (k_slab_split) the launch clears the keys, before k_peak_finish reads it
   SlabArgs a{};
   a.rden = rden;
   a.rden_div = rden_div;
