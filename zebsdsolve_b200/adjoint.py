@@ -136,8 +136,9 @@ def refine6(plan, q0, trust, most=60, gradient="reference"):
     parts = torch.empty((n + 31) // 32, 3, dtype=torch.float64, device=dev)
 
     def step(first):
-        # the sums at (x, qf), then the round's verdicts and the next (x, qf)
-        N.call("zeb_settle6", ptr(plan.run(mode, x, qf)), width, n, float(trust), first, ptr(state), ptr(x), ptr(qf),
+        # the sums at (x, qf), held until the call that reads them, then the round's verdicts and the next (x, qf)
+        sums = plan.run(mode, x, qf)
+        N.call("zeb_settle6", ptr(sums), width, n, float(trust), first, ptr(state), ptr(x), ptr(qf),
                ptr(parts), stream_ptr())
 
     step(1)
