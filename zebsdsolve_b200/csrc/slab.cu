@@ -30,6 +30,7 @@ struct SlabArgs {
   float2* cand;  // [item][nb]: (value, bits of index); keyed: (~index, ordered value) as one 64-bit key
   int keyed;
   float* vol;    // volume mode: [item][nb][nc][n]
+  int cols;      // columns a block of k_slab takes: nc, or in volume mode as many of them as fit
 };
 
 template <bool VOLUME>
@@ -38,19 +39,21 @@ __global__ void __launch_bounds__(256) k_slab(SlabArgs a) {
   __shared__ float redv[8];
   __shared__ uint32_t redi[8];
   const zeb_so3_dims_t& d = a.d;
-  const int L = d.L, nc = d.nc, n = d.n, nb = d.nb;
+  const int L = d.L, nc = VOLUME ? a.cols : d.nc, n = d.n, nb = d.nb;
   const int h = n >> 1;
-  const int slab = blockIdx.x;  // b·nb + j
+  const int groups = VOLUME ? d.nc / nc : 1;
+  const int slab = blockIdx.x / groups;  // b·nb + j
+  const int c0 = (blockIdx.x - slab * groups) * nc;
   const int b = slab / nb, j = slab - b * nb;
   const int lgc = a.lgc, lgh = a.lgh;
   float2* V = sm2;            // [L][nc]
   float2* Z = sm2 + L * nc;   // [h][nc]
   RowLines rows{lgc};
   ColLines cols{lgc};
-  const float2* src = a.U + (size_t)slab * L * nc;
+  const float2* src = a.U + (size_t)slab * L * d.nc + c0;
   for (int e = threadIdx.x; e < L * nc; e += blockDim.x) {
     int r = e >> lgc, c = e & (nc - 1);
-    V[rows(r, c)] = src[e];
+    V[rows(r, c)] = src[(size_t)r * d.nc + c];
   }
   __syncthreads();
   // Z down each column, bit-reversed along a
@@ -74,7 +77,7 @@ __global__ void __launch_bounds__(256) k_slab(SlabArgs a) {
   fft_lines_smem_lf(Z, nc, lgh, a.tw, cols);
 
   if (VOLUME) {
-    float* out = a.vol + (size_t)slab * nc * n;
+    float* out = a.vol + ((size_t)slab * d.nc + c0) * n;
     for (int e = threadIdx.x; e < nc * h; e += blockDim.x) {
       int c = e / h, p = e - c * h;
       float2 z = Z[cols(c, p)];
@@ -754,8 +757,16 @@ static bool dims_ok(const zeb_so3_dims_t* d) {
          d->n <= ZEB_TW_LEN;
 }
 
-static size_t slab_smem(const zeb_so3_dims_t* d) {
-  return ((size_t)d->L * d->nc + (size_t)(d->n / 2) * d->nc) * sizeof(float2);
+// shared memory of k_slab for `cols` columns
+static size_t slab_smem(const zeb_so3_dims_t* d, int cols) {
+  return ((size_t)d->L * cols + (size_t)(d->n / 2) * cols) * sizeof(float2);
+}
+constexpr size_t kSlabSmem = 220 * 1024;
+
+// slabs of these sizes take the block-wide split, whatever their columns: 128-point columns by 32, 128
+// columns of 64 points
+static bool slab_splits(const zeb_so3_dims_t* d) {
+  return (d->n == 256 && d->nc % 32 == 0) || (d->n == 128 && d->nc == 128);
 }
 
 }  // namespace zeb
@@ -792,12 +803,16 @@ static int slab_launch(const float* U, int n_items, const zeb_so3_dims_t* d, con
   a.U = (const float2*)U;
   a.n_items = n_items;
   a.d = *d;
-  a.lgc = ilog2i(d->nc);
+  // k_slab's columns: all of a slab, or, for the volume of a slab whose peaks the split kernel takes, as
+  // many as fit (each column's transform is its own)
+  a.cols = d->nc;
+  while (vol && slab_splits(d) && slab_smem(d, a.cols) > kSlabSmem) a.cols >>= 1;
+  a.lgc = ilog2i(a.cols);
   a.lgh = ilog2i(d->n / 2);
   a.tw = (const float2*)tw;
-  size_t smem = slab_smem(d);
-  ZEB_REQUIRE(smem <= 220 * 1024, ZEB_ESIZE, "correlate: slab of L=%d, nc=%d needs %zu bytes of shared memory", d->L,
-              d->nc, smem);
+  const size_t smem = slab_smem(d, a.cols);
+  ZEB_REQUIRE(smem <= kSlabSmem || slab_splits(d), ZEB_ESIZE,
+              "correlate: slab of L=%d, nc=%d needs %zu bytes of shared memory", d->L, d->nc, smem);
   long long blocks = (long long)n_items * d->nb;
   ZEB_REQUIRE(blocks < (1LL << 31), ZEB_ESIZE, "correlate: too many slabs");
   if (!vol && d->L <= d->n / 2) {
@@ -851,10 +866,11 @@ static int slab_launch(const float* U, int n_items, const zeb_so3_dims_t* d, con
     // split; items: k_slab → split: L = 128, nc = 64: 256 10.11 → 0.75 ms, 1 0.087 → 0.036; L = 80, nc = 128:
     // 128 9.45 → 0.61, 1 0.131 → 0.043; L = 64, nc = 128: 512 9.68 → 0.63, 1 0.085 → 0.031. Not fewer columns
     // of 64 points (nc = 32, 4096: 1.10 → 1.25).
-    if (H == 128 && NC % 32 == 0) return split_launch<16, 8, 3>(a, sms, st);
-    if (H == 64 && NC == 128) return split_launch<8, 8, 4>(a, sms, st);
+    if (slab_splits(d)) return H == 128 ? split_launch<16, 8, 3>(a, sms, st) : split_launch<8, 8, 4>(a, sms, st);
   }
   if (vol) {
+    blocks *= d->nc / a.cols;
+    ZEB_REQUIRE(blocks < (1LL << 31), ZEB_ESIZE, "correlate: too many slabs");
     cudaFuncSetAttribute(k_slab<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     k_slab<true><<<(unsigned)blocks, 256, smem, st>>>(a);
   } else {
