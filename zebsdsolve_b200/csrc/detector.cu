@@ -581,6 +581,10 @@ static size_t det_smem(DetArgs& a) {
 // 1.19 → 1.14; 1024 of 120 × 160 1.37 → 1.20 and 1.22 → 0.94. (Eight items of 128 threads with two pixels
 // in flight a thread instead of four: 4.48 and 3.39, but 300 patterns 0.191 → 0.234.)
 
+// The longest list these take: longer ones are zeb_refine's, whose records (other orders of the sums, FP32
+// lookups in either form) large detectors have always had. The kernel itself would fit twice as many.
+constexpr int RL_PIXELS = 25600;
+
 // the block size for a list of npix pixels: a longer one leaves fewer items an SM
 inline int rl_threads(int npix) { return npix <= 4608 ? 128 : (npix <= 9216 ? 256 : 512); }
 
@@ -867,9 +871,7 @@ extern "C" int zeb_refine_list(const float* pats, const float* items, const floa
               ZEB_EARG, "refine_list: bad arguments");
   ZEB_REQUIRE(fr && npix == zeb_mask_count(fr), ZEB_EARG, "refine_list: %d pixels listed, the frame masks %d", npix,
               fr ? zeb_mask_count(fr) : -1);
-  const size_t smem = (size_t)npix * 2 * sizeof(float);
-  ZEB_REQUIRE(npix >= 1 && smem <= DET_LIST_SMEM, ZEB_ESIZE, "refine_list: %d pixels (at most %zu)", npix,
-              DET_LIST_SMEM / 8);
+  ZEB_REQUIRE(npix >= 1 && npix <= RL_PIXELS, ZEB_ESIZE, "refine_list: %d pixels (at most %d)", npix, RL_PIXELS);
   if (n <= 0) return ZEB_OK;
   DetArgs a{};
   ZEB_REQUIRE(fill_frame(a, fr), ZEB_EARG, "refine_list: bad frame");
@@ -892,9 +894,7 @@ extern "C" int zeb_refine_list_h(const float* pats, const float* items, const fl
               ZEB_EARG, "refine_list_h: bad arguments");
   ZEB_REQUIRE(fr && npix == zeb_mask_count(fr), ZEB_EARG, "refine_list_h: %d pixels listed, the frame masks %d", npix,
               fr ? zeb_mask_count(fr) : -1);
-  const size_t smem = (size_t)npix * 2 * sizeof(float);
-  ZEB_REQUIRE(npix >= 1 && smem <= DET_LIST_SMEM, ZEB_ESIZE, "refine_list_h: %d pixels (at most %zu)", npix,
-              DET_LIST_SMEM / 8);
+  ZEB_REQUIRE(npix >= 1 && npix <= RL_PIXELS, ZEB_ESIZE, "refine_list_h: %d pixels (at most %d)", npix, RL_PIXELS);
   if (n <= 0) return ZEB_OK;
   DetArgs a{};
   ZEB_REQUIRE(fill_frame(a, fr), ZEB_EARG, "refine_list_h: bad frame");

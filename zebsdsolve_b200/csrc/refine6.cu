@@ -750,6 +750,7 @@ extern "C" int zeb_det6_list(int mode, const float* pats, const float* items, in
               "det6_list: pair tables misaligned");
   ZEB_REQUIRE(npix == zeb_mask_count(fr), ZEB_EARG, "det6_list: %d pixels listed, the frame masks %d", npix,
               zeb_mask_count(fr));
+  // (the entry points' own limit, and the plane fit's; the kernel keeps nothing a pixel)
   ZEB_REQUIRE(npix >= 1 && npix <= 51200, ZEB_ESIZE, "det6_list: %d pixels (at most 51200)", npix);
   if (n <= 0) return ZEB_OK;
   Det6Args a{};

@@ -1206,7 +1206,8 @@ class Engine:
 
     def mask_list(self, fr):
         """The frame's masked pixels in raster order on the device (zeb_mask_list), cached per
-        frame; None when the list is beyond the list kernel (zeb_refine then takes the frame)."""
+        frame; None when the list is longer than zeb_refine_list takes (zeb_refine and zeb_det6 then
+        take the frame)."""
         key = (fr.h, fr.w, tuple(fr.mask))
         hit = getattr(self, "_mask_list", None)
         if hit is not None and hit[0] == key:
@@ -1382,8 +1383,6 @@ class Engine:
         fr = self.frame()
         _, sheets, grad, vpair, gpair = self.phases[phase].baked
         lst = self.mask_list(fr)
-        if lst is not None and lst.numel() > 51200:
-            lst = None
         plan = adjoint.Plan(pats, items, fr, vpair, gpair, self.phases[phase].master.side, lst)
         s = self.set
         trust_px = (s["plane_trust"] if trust is None else float(trust)) * h
