@@ -111,3 +111,83 @@ def test_two_rounds(n, width):
     _, _, qn, sn = _trial(adjoint, torch.where(better[:, None], s2, s1), q, shift, lam, trust)
     assert near(state[33:36].t(), shift, 1e-15)
     assert near(state[37:41].t(), qn, 1e-8) and near(state[41:44].t(), sn, 1e-8)
+
+
+@pytest.mark.parametrize("width", [43, 61])
+def test_damping_at_its_bounds_and_small_rotations(width):
+    """λ set by hand before a round that keeps or loses the trial: it stays within [1e-4, 1e8], a loss at 1e8 is no
+    longer counted as damped, and at 1e8 the next step's rotation is far below the 1e-6 where its sine's series
+    takes over. The systems are then all but diagonal: a step is right to 1e-10 of its size, and a trial beside
+    it to the rounding of a unit quaternion, 2e-15."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from zebsdsolve_b200 import _native as N
+    from zebsdsolve_b200 import adjoint
+
+    n, trust = 96, 0.05
+    g = torch.Generator(device="cuda")
+    g.manual_seed(width)
+    s1, s2 = _sums(n, width, g), _sums(n, width, g)
+    state = torch.zeros(N.ZEB_SETTLE6_STATE, n, dtype=F64, device="cuda")
+    state[29:33] = torch.randn(4, n, generator=g, dtype=F64, device="cuda")
+    x, qf = torch.zeros(n, 6, device="cuda"), torch.zeros(n, 4, device="cuda")
+    parts = torch.empty((n + 31) // 32, 3, dtype=F64, device="cuda")
+
+    def step(s, first):
+        N.call("zeb_settle6", _p(s), width, n, trust, first, _p(state), _p(x), _p(qf), _p(parts),
+               ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+        torch.cuda.synchronize()
+
+    step(s1, 1)
+    given = torch.tensor([1e-4, 2e-4, 3e7, 1e8], dtype=F64, device="cuda").repeat(n // 4)
+    state[36] = given
+    was, q, qt, st = state[0].clone(), state[29:33].t().clone(), state[37:41].t().clone(), state[41:44].t().clone()
+    step(s2, 0)
+    _, ncc, _, _ = adjoint.local_of(s2[:, :43])
+    better = ncc > was
+    assert 4 <= int(better.sum()) <= n - 4
+    lam = torch.where(better, (given / 3).clamp(min=1e-4), (given * 5).clamp(max=1e8))
+    assert torch.equal(state[36], lam)
+    _, kept, damp = parts.sum(0).tolist()
+    assert kept == int(better.sum()) and damp == int((~better & (given < 1e8)).sum())
+    q, shift = torch.where(better[:, None], qt, q), torch.where(better[:, None], st, 0 * st)
+    _, _, qn, sn = _trial(adjoint, torch.where(better[:, None], s2, s1), q, shift, lam, trust)
+    small = lam >= 1e7
+    d = 2 * (qn - q)[small].norm(dim=1)
+    assert int(small.sum()) >= 40 and float(d.max()) < 1e-6
+    assert bool(((state[37:41].t() - qn)[small].abs() <= 1e-10 * d[:, None] + 2e-15).all())
+    assert bool(((state[41:44].t() - sn)[small].abs() <= 1e-10 * (sn - shift)[small].abs() + 1e-17).all())
+
+
+def test_solve6():
+    """Random systems, some with a pivot that has to be fetched from another row, some singular, one with a NaN: the
+    residual is the rounding of an elimination with partial pivoting, 6^2 · 2^-52 (|A||x| + |b|) with room for the
+    growth of 6 pivots (2^5)."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from zebsdsolve_b200 import _native as N
+
+    n = 300
+    g = torch.Generator(device="cuda")
+    g.manual_seed(5)
+    A = torch.randn(n, 6, 6, generator=g, dtype=F64, device="cuda")
+    A[1::5, 0, 0] = 0
+    A[2::5, 2:4, 2] = 0
+    A[3::5, :, 4] = 0  # singular
+    A[4] = 0
+    A[9, 3, 3] = float("nan")
+    b = torch.randn(n, 6, generator=g, dtype=F64, device="cuda")
+    x = torch.full((n, 6), 7.0, dtype=F64, device="cuda")
+    ok = torch.full((n,), -1, dtype=torch.int32, device="cuda")
+    N.call("zeb_solve6", _p(A), _p(b), n, _p(x), _p(ok), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    want = torch.ones(n, dtype=torch.int32, device="cuda")
+    want[3::5] = 0
+    want[4] = 0
+    assert torch.equal(ok, want) and bool((x[ok == 0] == 0).all()) and bool(torch.isnan(x[9]).any())
+    use = ok != 0
+    use[9] = False
+    A, b, x = A[use], b[use], x[use]
+    off = (torch.einsum("nij,nj->ni", A, x) - b).abs()
+    bound = 36 * 32 * 2.0 ** -52 * (torch.einsum("nij,nj->ni", A.abs(), x.abs()) + b.abs()).amax(1, keepdim=True)
+    assert bool((off <= bound).all())

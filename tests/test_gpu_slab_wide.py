@@ -2,7 +2,7 @@
 fold): the volume by groups of columns against a float64 inverse FFT, and a two-fold master indexed at L = 128
 (GPU only).
 
-Tolerance of the volume: as test_gpu_slab_split, 2 (log2 n + 2) 2^-24 of its column's 2 Σ|V|; of the orientations:
+Tolerance of the volume: as slab_calls has it, 2 (log2 n + 2) 2^-24 of its column's 2 Σ|V|; of the orientations:
 test_gpu_configs' for the same bandwidth.
 """
 import ctypes
@@ -11,56 +11,51 @@ import tempfile
 
 import numpy as np
 import pytest
-import test_gpu_slab_split as split
 
 torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("L,fold,n", [(93, 2, 2), (128, 2, 3), (65, 1, 2), (128, 1, 1), (92, 2, 1), (64, 1, 2)])
-def test_the_volume_of_a_wide_slab(L, fold, n):
+@pytest.fixture(autouse=True)
+def device():
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")
-    from zebsdsolve_b200 import _native as N
 
-    d = split._dims(L, fold)
-    g = torch.Generator(device="cuda")
-    g.manual_seed(L + fold)
-    U = torch.randn(n, d.nb, L, d.nc, 2, device="cuda", generator=g)
-    count, guard = n * d.nb * d.nc * d.n, 4096
-    vol = torch.full((count + guard,), 9.0, device="cuda")
-    N.call("zeb_correlate_volume", split._p(U), n, ctypes.byref(d), split._p(split._tw()), split._p(vol), split._sp())
-    assert bool((vol[count:] == 9.0).all())
-    V = torch.view_as_complex(U.double()).transpose(2, 3)  # [b][j][c][m']
-    pad = torch.zeros(n, d.nb, d.nc, d.n // 2 + 1, dtype=torch.complex128, device="cuda")
-    pad[..., :L] = V.conj()
-    want = torch.fft.irfft(pad, n=d.n, dim=-1) * d.n
-    tol = 2 * (math.log2(d.n) + 2) * 2.0 ** -24 * 2 * V.abs().sum(-1, keepdim=True)
-    assert bool(((vol[:count].view_as(want).double() - want).abs() <= tol).all())
+
+@pytest.mark.parametrize("L,fold,n", [(93, 2, 2), (128, 2, 3), (65, 1, 2), (128, 1, 1), (92, 2, 1), (64, 1, 2)])
+def test_the_volume_of_a_wide_slab(L, fold, n):
+    import slab_calls as sc
+
+    d, U, _ = sc.inputs(L, fold, n, 1 << 30, L + fold)
+    vol, past = sc.volume(U, n, d, guard=4096)
+    assert bool((past == 9.0).all())
+    want, size = sc.exact_volume(U, d)
+    tol = 2 * (math.log2(d.n) + 2) * 2.0 ** -24 * 2 * size[..., None]
+    assert bool(((vol.double() - want).abs() <= tol).all())
 
 
 @pytest.mark.parametrize("L,fold,n,div", [(128, 2, 3, 1 << 30), (93, 2, 4, 2), (65, 1, 2, 1)])
 def test_the_peaks_of_a_wide_slab(L, fold, n, div):
-    split.test_split_transform_gives_the_shared_memory_transform_s_bits(L, fold, n, div)
+    import slab_calls as sc
+
+    d, U, rden = sc.inputs(L, fold, n, div, L * 16 + fold)
+    sc.check_split_bits(U, rden, n, d, div)
 
 
 def test_slabs_without_a_split_stay_refused():
-    if not torch.cuda.is_available():
-        pytest.skip("no CUDA device")
+    import slab_calls as sc
     from zebsdsolve_b200 import _native as N
 
     x = torch.zeros(64, device="cuda")
-    d = split._dims(160, 4)  # 256-point columns, 128 of them
-    for call in (lambda: N.call("zeb_correlate_volume", split._p(x), 1, ctypes.byref(d), split._p(x), split._p(x), split._sp()),
-                 lambda: split._peaks(x, 1, d, x, 1)):
-        with pytest.raises(N.NativeError, match="shared memory"):
-            call()
+    d = sc.dims(160, 4)  # 256-point columns, 128 of them
+    with pytest.raises(N.NativeError, match="shared memory"):
+        N.call("zeb_correlate_volume", sc.ptr(x), 1, ctypes.byref(d), sc.ptr(x), sc.ptr(x), sc.stream())
+    with pytest.raises(N.NativeError, match="shared memory"):
+        sc.peaks(x, 1, d, x, 1)
 
 
 @pytest.mark.parametrize("precision", ["f32", "bf16"])
 def test_a_two_fold_master_at_bandwidth_128(precision):
-    if not torch.cuda.is_available():
-        pytest.skip("no CUDA device")
     import zebsdsolve_b200 as ze
     from zebsdsolve_b200 import synthetic as syn
     from zebsdsolve_b200.master import write_npz
