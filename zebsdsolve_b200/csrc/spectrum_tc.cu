@@ -132,10 +132,12 @@ __global__ void k_pack_master(const double2* __restrict__ Y, TcLayout t, int mp,
 }
 
 // B_m'[b][κ] from the coefficients (complex f32 [b][pair]): a block per (K-block, pattern tile, order;
-// `most` K-blocks or fewer an order), a thread per 16-byte chunk of four rows (a chunk is four degrees'
-// re and im, of one segment or two). It moves 3 × n_pairs × 8 bytes an item, little beside the spectrum
-// it feeds: a thread per chunk with its own division and its own walk over the lower orders' sizes
-// made it 14 % of the two, 0.815 → 0.758 ms with this split (6144 items, L = 64, nc = 32).
+// `most` K-blocks or fewer an order; and half of the tile's rows), a thread per 16-byte chunk of two rows
+// (a chunk is four degrees' re and im, of one segment or two). It moves 3 × n_pairs × 8 bytes an item,
+// little beside the spectrum it feeds: a thread per chunk with its own division and its own walk over the
+// lower orders' sizes made it 14 % of the two, 0.815 → 0.758 ms with this split (6144 items, L = 64, nc = 32).
+// Two rows a thread and not four: as fast for many items (3072: 0.403 ms) and for few the chain of loads is
+// shorter (the two kernels, 128 items: L = 64 64 → 61 µs, L = 32 25 → 23, L = 16 20 → 18).
 __global__ void __launch_bounds__(256) k_pack_patterns(const float2* __restrict__ alm, int n_items, int n_pairs,
                                                        TcLayout t, int most, uint8_t* __restrict__ B) {
   const int ptile = blockIdx.x / most, kblock = blockIdx.x - ptile * most, mp = blockIdx.y;
@@ -150,8 +152,8 @@ __global__ void __launch_bounds__(256) k_pack_patterns(const float2* __restrict_
   const int n0 = tc_k0(t.L, mp) >> 1, n1 = tc_k1(t.L, mp, t.split) >> 1;  // degrees of segment 0, of 1 and 2
   const int c16 = threadIdx.x & 7;
 #pragma unroll
-  for (int it = 0; it < 4; ++it) {
-    const int row = (threadIdx.x >> 3) + 32 * it, b = ptile * TC_BN + row;
+  for (int it = 0; it < 2; ++it) {
+    const int row = (threadIdx.x >> 3) + 32 * (2 * blockIdx.z + it), b = ptile * TC_BN + row;
     const float2* src = alm + (size_t)b * n_pairs + p0;
     uint32_t v[4];
 #pragma unroll
@@ -519,7 +521,7 @@ extern "C" int zeb_spectrum_bf16(const float* alm, int n_items, const zeb_so3_di
   cudaStream_t st = (cudaStream_t)stream;
   int most = 1;  // (an order's K-blocks do not grow with it)
   for (int mp = 0; mp < d->L; ++mp) most = std::max(most, tc_kblocks(d->L, mp, split));
-  const dim3 gp((unsigned)most * t.ptiles, d->L);
+  const dim3 gp((unsigned)most * t.ptiles, d->L, TC_BN / 64);
   k_pack_patterns<<<gp, 256, 0, st>>>((const float2*)alm, n_items, d->n_pairs, t, most, (uint8_t*)B);
   int rc = zeb_launch_check("pack_patterns");
   if (rc) return rc;
@@ -591,7 +593,7 @@ extern "C" int zeb_spectrum_bf16_h(const float* alm, int n_items, const zeb_so3_
   cudaStream_t st = (cudaStream_t)stream;
   int most = 1;  // (an order's K-blocks do not grow with it)
   for (int mp = 0; mp < d->L; ++mp) most = std::max(most, tc_kblocks(d->L, mp, split));
-  const dim3 gp((unsigned)most * t.ptiles, d->L);
+  const dim3 gp((unsigned)most * t.ptiles, d->L, TC_BN / 64);
   k_pack_patterns<<<gp, 256, 0, st>>>((const float2*)alm, n_items, d->n_pairs, t, most, (uint8_t*)B);
   int rc = zeb_launch_check("pack_patterns");
   if (rc) return rc;
