@@ -580,6 +580,12 @@ static size_t det_smem(DetArgs& a) {
 // 16384 patterns of 60 × 60 4.95 → 4.51 ms in FP32, 3.71 → 3.37 in FP16; 2048 of 96 × 96 1.61 → 1.48 and
 // 1.19 → 1.14; 1024 of 120 × 160 1.37 → 1.20 and 1.22 → 0.94. (Eight items of 128 threads with two pixels
 // in flight a thread instead of four: 4.48 and 3.39, but 300 patterns 0.191 → 0.234.)
+//
+// FEW: patterns too few to fill the SMs so gain nothing from more of them an SM, and the long lists' kernels pay
+// for those with registers (two pixels in flight a thread). They keep four in flight, at three blocks of 256
+// threads an SM, or one of 512, whose shared memory then has room for the pattern's values too. Many → few, at
+// 96 × 96 (256 threads) 148 patterns 263 → 218 µs in FP32 and 221 → 204 in FP16, 740 694 → 623 and 501 → 468;
+// at 120 × 160 (512) 148 patterns 273 → 228 and 213 → 201.
 
 // The longest list these take: longer ones are zeb_refine's, whose records (other orders of the sums, FP32
 // lookups in either form) large detectors have always had. The kernel itself would fit twice as many.
@@ -587,6 +593,16 @@ constexpr int RL_PIXELS = 25600;
 
 // the block size for a list of npix pixels: a longer one leaves fewer items an SM
 inline int rl_threads(int npix) { return npix <= 4608 ? 128 : (npix <= 9216 ? 256 : 512); }
+
+// whether n patterns take the FEW form on a GPU of `sms` SMs. 512 threads: while a block an SM holds them all (at
+// 120 × 160 297 patterns already take 366 µs in the other form against 422). 256 threads: where three blocks an
+// SM need no more time in their waves than four do in theirs, a wave of four taking 1.3 times one of three (520
+// patterns of 96 × 96: 440 µs against 545 the other way); past six a SM the waves have run into one another.
+inline bool rl_few(int n, int th, int sms) {
+  if (th == 512) return n <= sms;
+  const int w3 = (n + 3 * sms - 1) / (3 * sms), w4 = (n + 4 * sms - 1) / (4 * sms);
+  return n <= 6 * sms && w3 * 10 < w4 * 13;
+}
 
 __device__ __forceinline__ float3 list_ray(const DetArgs& a, float3 t, uint32_t v) {
   return ray_dir(a, t, (int)(v >> 16), (int)(v & 0xffffu));
@@ -597,14 +613,15 @@ __device__ __forceinline__ float list_value(const DetArgs& a, const float* __res
 }
 
 // the NMI over the list (detector.wgsl:744-832) of the pattern gpat; sims (shared, npix floats) keeps the
-// simulated values of the first pass for the histogram pass
+// simulated values of the first pass for the histogram pass. STAGED: the pattern's values lie behind them
+template <bool STAGED>
 __device__ float nmi_list(const DetArgs& a, const uint32_t* __restrict__ list, const float* __restrict__ gpat, float* sims,
                           int npix, float3 t, float4 q, int nbins, uint32_t* hist, float* red) {
   float ext[4] = {3.4e38f, -3.4e38f, 3.4e38f, -3.4e38f};
 #pragma unroll 4
   for (int k = threadIdx.x; k < npix; k += blockDim.x) {
     const uint32_t v = __ldg(list + k);
-    const float e = list_value(a, gpat, v);
+    const float e = STAGED ? sims[npix + k] : list_value(a, gpat, v);
     const float sv = master_at_pair(a.vpair, qrot(q, list_ray(a, t, v)), a.side);
     sims[k] = sv;
     ext[0] = fminf(ext[0], e); ext[1] = fmaxf(ext[1], e);
@@ -631,8 +648,8 @@ __device__ float nmi_list(const DetArgs& a, const uint32_t* __restrict__ list, c
   const float ke = (float)nbins / fmaxf(r[1] - r[0], 1e-20f);
   const float ks = (float)nbins / fmaxf(r[3] - r[2], 1e-20f);
   for (int k = threadIdx.x; k < npix; k += blockDim.x) {
-    const uint32_t v = __ldg(list + k);
-    const uint32_t be = min((uint32_t)((list_value(a, gpat, v) - r[0]) * ke), (uint32_t)(nbins - 1));
+    const float e = STAGED ? sims[npix + k] : list_value(a, gpat, __ldg(list + k));
+    const uint32_t be = min((uint32_t)((e - r[0]) * ke), (uint32_t)(nbins - 1));
     const uint32_t bs = min((uint32_t)((sims[k] - r[2]) * ks), (uint32_t)(nbins - 1));
     atomicAdd(&hist[be * nbins + bs], 1u);
   }
@@ -667,10 +684,11 @@ struct RefineState {
 // QUAD: the lookups from the FP16 neighbourhood records (a.gpair holds zeb_master_quads' table)
 // TH threads a pattern: 128 (seven patterns an SM) while the list is small; a long list takes 256 or
 // 512, so that its serial phases stay short beside its passes
-template <bool QUAD, int TH>
-__global__ void __launch_bounds__(TH, TH == 128 ? 7 : (TH == 256 ? 4 : 2))
+template <bool QUAD, int TH, bool FEW>
+__global__ void __launch_bounds__(TH, TH == 128 ? 7 : (TH == 256 ? (FEW ? 3 : 4) : (FEW ? 1 : 2)))
     k_refine_list(DetArgs a, const uint32_t* __restrict__ list, int npix) {
-  extern __shared__ float sims[];  // [npix] simulated values (NMI)
+  constexpr bool STAGED = FEW && TH == 512;
+  extern __shared__ float sims[];  // [npix] simulated values (NMI); STAGED: then [npix] pattern values
   __shared__ float red[20 * (TH / 32)];
   __shared__ uint32_t hist[32 * 32];
   __shared__ float4 sh_q;
@@ -690,6 +708,8 @@ __global__ void __launch_bounds__(TH, TH == 128 ? 7 : (TH == 256 ? 4 : 2))
     st.mu = a.o.scale0;
     sh_q = st.q_best;
   }
+  if (STAGED)
+    for (int k = threadIdx.x; k < npix; k += TH) sims[npix + k] = list_value(a, gpat, __ldg(list + k));
   __syncthreads();
 
   for (int iter = 0; iter <= a.o.iters; ++iter) {
@@ -699,7 +719,7 @@ __global__ void __launch_bounds__(TH, TH == 128 ? 7 : (TH == 256 ? 4 : 2))
     float s[19];
 #pragma unroll
     for (int k = 0; k < 19; ++k) s[k] = 0.f;
-#pragma unroll (TH == 128 ? 4 : 2)
+#pragma unroll (TH == 128 || FEW ? 4 : 2)
     for (int k = threadIdx.x; k < npix; k += TH) {
       const uint32_t v = __ldg(list + k);
       const float row = (float)(int)(v >> 16), col = (float)(int)(v & 0xffffu);
@@ -708,7 +728,7 @@ __global__ void __launch_bounds__(TH, TH == 128 ? 7 : (TH == 256 ? 4 : 2))
                                               fmaf(rc0.z, row, fmaf(rc1.z, col, rt.z))));
       const float4 m = QUAD ? grad_at_quad(a.gpair, c, a.side) : grad_at_pair(a.gpair, c, a.side);
       const float3 d = cross3(c, make_float3(m.x, m.y, m.z));
-      const float e = list_value(a, gpat, v);
+      const float e = STAGED ? sims[npix + k] : list_value(a, gpat, v);
       s[1] += m.w; s[2] += m.w * m.w; s[3] += m.w * e;
       s[4] += d.x; s[5] += d.y; s[6] += d.z;
       s[7] += m.w * d.x; s[8] += m.w * d.y; s[9] += m.w * d.z;
@@ -766,7 +786,7 @@ __global__ void __launch_bounds__(TH, TH == 128 ? 7 : (TH == 256 ? 4 : 2))
     __syncthreads();
   }
   const float4 qf = sh_q;
-  const float v = nmi_list(a, list, gpat, sims, npix, t, qf, a.o.nmi_bins, hist, red);
+  const float v = nmi_list<STAGED>(a, list, gpat, sims, npix, t, qf, a.o.nmi_bins, hist, red);
   if (threadIdx.x == 0) {
     float* r = a.records + (size_t)b * 8;
     r[0] = qf.x; r[1] = qf.y; r[2] = qf.z; r[3] = qf.w;
@@ -799,20 +819,24 @@ __global__ void k_mask_list(DetArgs a, uint32_t* __restrict__ list) {
   }
 }
 
-template <bool QUAD, int TH>
-void rl_launch_th(const DetArgs& a, const uint32_t* list, int npix, cudaStream_t st) {
-  const size_t smem = (size_t)npix * sizeof(float);
+template <bool QUAD, int TH, bool FEW>
+void rl_launch_as(const DetArgs& a, const uint32_t* list, int npix, cudaStream_t st) {
+  const size_t smem = (size_t)npix * sizeof(float) * (FEW && TH == 512 ? 2 : 1);
   if (smem > 40 * 1024)  // (beside the static 5 KB)
-    cudaFuncSetAttribute(k_refine_list<QUAD, TH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  k_refine_list<QUAD, TH><<<a.n, TH, smem, st>>>(a, list, npix);
+    cudaFuncSetAttribute(k_refine_list<QUAD, TH, FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  k_refine_list<QUAD, TH, FEW><<<a.n, TH, smem, st>>>(a, list, npix);
 }
 
 template <bool QUAD>
 void rl_launch(const DetArgs& a, const uint32_t* list, int npix, cudaStream_t st) {
   const int th = rl_threads(npix);
-  if (th == 128) rl_launch_th<QUAD, 128>(a, list, npix, st);
-  else if (th == 256) rl_launch_th<QUAD, 256>(a, list, npix, st);
-  else rl_launch_th<QUAD, 512>(a, list, npix, st);
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const bool few = rl_few(a.n, th, sms);
+  if (th == 128) rl_launch_as<QUAD, 128, false>(a, list, npix, st);
+  else if (th == 256) few ? rl_launch_as<QUAD, 256, true>(a, list, npix, st) : rl_launch_as<QUAD, 256, false>(a, list, npix, st);
+  else few ? rl_launch_as<QUAD, 512, true>(a, list, npix, st) : rl_launch_as<QUAD, 512, false>(a, list, npix, st);
 }
 
 }  // namespace zeb
