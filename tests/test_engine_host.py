@@ -73,3 +73,51 @@ def test_a_first_sweep_pass_lands_as_slices():
     for k in fast.res:
         assert np.array_equal(fast.res[k][10:30], slow.res[k][10:30]), k
     assert fast.index_accepted == slow.index_accepted and fast.index_done == slow.index_done == 20
+
+
+@pytest.mark.parametrize("rows,cols,radius,passes", [(1, 1, 1, 1), (5, 7, 1, 3), (9, 4, 3, 2), (6, 11, 2, 1)])
+def test_an_averaging_window_s_neighbours(rows, cols, radius, passes):
+    """nbr by its definition, cell by cell: the list index of the cell at each offset, 0xffffffff outside the map or
+    the list (the frame around the map is never read as the map's other side)."""
+    e = _engine(rows, cols)
+    e.set.apply({"nlpar_radius": radius, "nlpar_iterations": passes})
+    reach = radius * passes
+    for wanted in (np.arange(rows * cols), np.arange(1), np.array([rows * cols - 1, 0])):
+        cells, counts, nbr = e.nlpar_window(wanted)
+        index = {int(c): k for k, c in enumerate(cells)}
+        assert len(index) == len(cells) == counts[-1] and counts[0] == len(np.unique(wanted))
+        want = np.full((len(cells), 2 * reach + 1, 2 * reach + 1), 0xFFFFFFFF, np.uint32)
+        for k, c in enumerate(cells):
+            for dy in range(-reach, reach + 1):
+                for dx in range(-reach, reach + 1):
+                    y, x = c // cols + dy, c % cols + dx
+                    if 0 <= y < rows and 0 <= x < cols and y * cols + x in index:
+                        want[k, dy + reach, dx + reach] = index[y * cols + x]
+        assert nbr.dtype == np.uint32 and np.array_equal(nbr, want.reshape(len(cells), -1))
+
+
+def test_an_averaging_s_report():
+    """The batch's mean noise, the share of it an average keeps and the pattern's own share, against the sums cell by
+    cell; a cell without noise is counted in the own share alone."""
+    e = _engine()
+    e.set.apply({"nlpar_radius": 1, "nlpar_iterations": 1})
+    said = []
+    e.log = said.append
+    rng = np.random.default_rng(8)
+    n, F = 7, 9
+    shares = rng.random(n * F + 5).astype(np.float32)
+    sig = rng.random(12).astype(np.float32)
+    sig[2] = 0
+    nbr = rng.integers(0, 12, (10, F)).astype(np.uint32)
+    nbr[1, :4] = 0xFFFFFFFF
+    e._log_nlpar(sig, shares, nbr, n, F)
+    noise = kept = own = 0.0
+    for c in range(n):
+        sh = shares[c * F:(c + 1) * F].astype(np.float64)
+        own += sh[F // 2]
+        if sig[c] > 0:
+            after = sum(s * s * float(sig[k]) for s, k in zip(sh, nbr[c]) if k != 0xFFFFFFFF)
+            noise += float(sig[c]) ** 0.5
+            kept += (after / float(sig[c])) ** 0.5
+    assert f"noise about {noise / 6:.2f} a pixel" in said[0]
+    assert f"{100 * kept / 6:.0f} % of it left; an average is {100 * own / 7:.0f} % the pattern" in said[0]
