@@ -26,8 +26,8 @@
 // TCH_STAGES for the FP16 one), warp 1 allocates TMEM and one of its threads issues the MMAs
 // (M = 128 rows of ν, N = 128 patterns, K = 16 a step) into two accumulators of 128 columns, warps
 // 2-5 drain an accumulator (tcgen05.ld) while the next one fills: the FP32 U 32 patterns at a time
-// through shared memory into a tensor store, the FP16 U a whole tile at once (scattered 128-byte
-// stores from four warps cap an SM near 13 GB/s; the tensor store does not). Every wait is
+// through shared memory into a tensor store, the FP16 U a whole tile at once (faster than
+// the drain warps' own scattered 128-byte stores). Every wait is
 // bounded: on a timeout the CTA records the failure, drains what it issued, frees its TMEM and
 // returns.
 #include <cuda.h>
